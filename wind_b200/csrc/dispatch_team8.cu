@@ -5,26 +5,14 @@
 
 namespace wind {
 
-using TeamFn = void (*)(KParams);
+using TeamFn = void (*)(KParams, int);
 
-template <int NMAX, int METHOD, int CTRL>
-static TeamFn team_by_solver(int solver) {
-    if constexpr (METHOD == WIND_METHOD_RK2) return k_team<NMAX, METHOD, CTRL, 0>;
-    else {
-        switch (solver) {
-        case WIND_SOLVER_GJE_F64: return k_team<NMAX, METHOD, CTRL, WIND_SOLVER_GJE_F64>;
-        case WIND_SOLVER_LU_F64: return k_team<NMAX, METHOD, CTRL, WIND_SOLVER_LU_F64>;
-        default: return k_team<NMAX, METHOD, CTRL, WIND_SOLVER_MIXED>;
-        }
-    }
-}
-
-TeamFn team_fn_8(int method, int ctrl, int solver) {
+TeamFn team_fn_8(int method, int ctrl) {
     if (method == WIND_METHOD_SIE)
-        return ctrl == WIND_CTRL_GOLD ? team_by_solver<8, WIND_METHOD_SIE, WIND_CTRL_GOLD>(solver)
-                                      : team_by_solver<8, WIND_METHOD_SIE, WIND_CTRL_DEVICE>(solver);
-    return ctrl == WIND_CTRL_GOLD ? team_by_solver<8, WIND_METHOD_RK2, WIND_CTRL_GOLD>(solver)
-                                  : team_by_solver<8, WIND_METHOD_RK2, WIND_CTRL_DEVICE>(solver);
+        return ctrl == WIND_CTRL_GOLD ? k_team<8, WIND_METHOD_SIE, WIND_CTRL_GOLD>
+                                      : k_team<8, WIND_METHOD_SIE, WIND_CTRL_DEVICE>;
+    return ctrl == WIND_CTRL_GOLD ? k_team<8, WIND_METHOD_RK2, WIND_CTRL_GOLD>
+                                  : k_team<8, WIND_METHOD_RK2, WIND_CTRL_DEVICE>;
 }
 
 }  // namespace wind

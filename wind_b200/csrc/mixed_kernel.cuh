@@ -19,6 +19,19 @@ namespace wind {
 
 constexpr int MIXED_THREADS = CTA_THREADS;
 
+// Teams of a block that run a group of the team kernel: all that the lanes
+// hold, or as many as the shared-memory budget does.
+__host__ __device__ inline int mixed_teams(int nmax, const TeamLayout& lay, int smem_cap) {
+    const int full = MIXED_THREADS / nmax, fit = smem_cap / lay.bytes;
+    return fit < full ? fit : full;
+}
+
+template <int NMAX, int METHOD, int CTRL>
+__device__ __forceinline__ void mixed_team_run(const KParams& p, unsigned char* smem_raw, int smem_cap) {
+    const TeamLayout lay(NMAX, p.n_react, p.linear != nullptr, METHOD == WIND_METHOD_SIE);
+    team_run<NMAX, METHOD, CTRL>(p, smem_raw, mixed_teams(NMAX, lay, smem_cap), 32 / NMAX);
+}
+
 // Two blocks per SM (128 registers) for the LU and mixed solvers, whose team
 // and CTA paths fit that budget; the reference Gauss-Jordan keeps a row of M
 // and of the inverse per lane in registers and gets the whole file.
@@ -39,9 +52,9 @@ __global__ void __launch_bounds__(MIXED_THREADS, SOLVER == WIND_SOLVER_GJE_F64 ?
                 else if (p.n_eq > 8) warp_run<16, CTRL, SMALL>(p, smem_raw);
                 else warp_run<8, CTRL, SMALL>(p, smem_raw);
             } else {
-                if (p.n_eq > 16) team_run<32, METHOD, CTRL, SOLVER>(p, smem_raw);
-                else if (p.n_eq > 8) team_run<16, METHOD, CTRL, SOLVER>(p, smem_raw);
-                else team_run<8, METHOD, CTRL, SOLVER>(p, smem_raw);
+                if (p.n_eq > 16) mixed_team_run<32, METHOD, CTRL>(p, smem_raw, smem_cap);
+                else if (p.n_eq > 8) mixed_team_run<16, METHOD, CTRL>(p, smem_raw, smem_cap);
+                else mixed_team_run<8, METHOD, CTRL>(p, smem_raw, smem_cap);
             }
         }
         __syncthreads();

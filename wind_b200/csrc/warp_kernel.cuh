@@ -39,9 +39,16 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "team_kernel.cuh"
 
 namespace wind {
+
+// Packed pivot key: |a| as float bits (low 5 mantissa bits replaced by the
+// inverted lane index, so ties go to the lowest lane), 0 for retired lanes.
+__device__ __forceinline__ unsigned pivot_key(double a, int lane_in_team, bool active) {
+    if (!active) return 0u;
+    const float m = fabsf((float)a);
+    return (__float_as_uint(m) & ~31u) | (31u - (unsigned)lane_in_team);
+}
 
 constexpr int WARP_THREADS = 128;
 constexpr int WARP_MIX_MAXIT = 8;     // refinement sweeps with a reused inverse
