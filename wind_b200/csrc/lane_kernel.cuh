@@ -24,20 +24,21 @@
 namespace wind {
 
 constexpr int LANE_THREADS = 128;
-// Minimum resident blocks per SM the compiler must plan registers for.  The
-// LU solver runs faster capped at 128 registers (4 blocks of 128 threads per
-// SM: 51-52 ms against 63-64 ms per 65,536-cell Katz96 call, measured back
-// to back on one B200, despite ~230 bytes of spills); the Gauss-Jordan path
-// loses under the same cap (600 -> 678 ms) and the mixed path was not
-// measured capped, so both keep the uncapped allocation.
+// Minimum resident blocks per SM the compiler must plan registers for: 4 (128
+// registers) for the FP64 solvers by blocks.  65,536 Katz96 cells with the LU
+// at atol 1e-8 / rtol 1e-6 took 42.0, 42.1, 43.2 and 47.1 ms at 3, 4, 5 and 6
+// (64.6 ms with the full-width 5 x 5 LU), 8,000 cells through the drop-in with
+// the Gauss-Jordan inverse 1.19, 1.17, 1.20 and 1.22 ms (2.87 ms full width).
+// The mixed path keeps the uncapped allocation.
 template <int SOLVER>
 struct LaneMinBlocks {
-    static constexpr int value = SOLVER == WIND_SOLVER_LU_F64 ? 4 : 1;
+    static constexpr int value = SOLVER == WIND_SOLVER_MIXED ? 1 : 4;
 };
 
-// One SIE or explicit-Euler substep of length h, in place on y.
+// One SIE or explicit-Euler substep of length h, in place on y, with the
+// full-width solvers.
 template <class Net, int METHOD, int CTRL, int SOLVER>
-__device__ __forceinline__ void lane_substep(const double (&c)[Net::NC], xd h, xd (&y)[Net::N]) {
+__device__ __forceinline__ void lane_substep_full(const double (&c)[Net::NC], xd h, xd (&y)[Net::N]) {
     constexpr int N = Net::N;
     xd f[N];
     Net::rhs(c, y, f);
@@ -130,6 +131,120 @@ __device__ __forceinline__ void lane_substep(const double (&c)[Net::NC], xd h, x
     lu_solve_reg<N, float, double>(Af, rinvf, perm, res);
 #pragma unroll
     for (int e = 0; e < N; e++) y[e] = y[e].v + h.v * (x[e] + res[e]);
+}
+
+// The same, out of line, for the substeps whose block solve met an infinite
+// or NaN value (a full-width elimination spreads those across blocks).
+template <class Net, int CTRL, int SOLVER>
+__device__ __noinline__ void lane_substep_redo(const double* c_in, double h, double* y_io) {
+    double c[Net::NC];
+    xd y[Net::N];
+#pragma unroll
+    for (int k = 0; k < Net::NC; k++) c[k] = c_in[k];
+#pragma unroll
+    for (int e = 0; e < Net::N; e++) y[e] = y_io[e];
+    lane_substep_full<Net, WIND_METHOD_SIE, CTRL, SOLVER>(c, xd(h), y);
+#pragma unroll
+    for (int e = 0; e < Net::N; e++) y_io[e] = y[e].v;
+}
+
+// The SIE substep of the diagonal block of size n at equation O, from the
+// system's f and Jt (both at the state in y): the stepped components go to
+// out, the high words of its pivots (GJE_F64) and results into hi.
+template <class Net, int CTRL, int SOLVER, int O, int n, bool TRI>
+__device__ __forceinline__ void lane_block_step(const xd (&Jt)[Net::N * Net::N], const xd (&f)[Net::N], xd h,
+                                                const xd (&y)[Net::N], xd (&out)[Net::N], int& hi) {
+    constexpr int N = Net::N;
+    if (SOLVER == WIND_SOLVER_GJE_F64) {
+        xd M[n * n], Inv[n * n];
+#pragma unroll
+        for (int i = 0; i < n; i++)
+#pragma unroll
+            for (int j = 0; j < n; j++) {
+                const xd e = Jt[(O + i) * N + O + j];
+                if (CTRL == WIND_CTRL_GOLD) {
+                    // sie_gold.c:17-36: J = -h*J; diag += 1
+                    M[i * n + j] = -h * e;
+                    if (i == j) M[i * n + j] += 1.0;
+                } else {
+                    // kernel.cu:49-52: J[i][j] = (i==j) - J[i][j]*h
+                    M[i * n + j] = xd(i == j ? 1.0 : 0.0) - e * h;
+                }
+            }
+        gje_invert_block<n, TRI>(M, Inv, hi);
+        if (CTRL == WIND_CTRL_GOLD) {
+            // matrix_ops.c:6-27 (transposed matvec), then sie_gold.c:72-74
+#pragma unroll
+            for (int r = 0; r < n; r++) {
+                xd acc = Inv[r] * f[O];
+#pragma unroll
+                for (int cc = 1; cc < n; cc++) acc += Inv[cc * n + r] * f[O + cc];
+                out[O + r] = y[O + r] + h * acc;
+            }
+        } else {
+            // kernel.cu:116-125: y_j += (Inv[k][j]*f_k)*h, k ascending
+#pragma unroll
+            for (int j = 0; j < n; j++) {
+                xd acc = y[O + j];
+#pragma unroll
+                for (int k = 0; k < n; k++) acc += Inv[k * n + j] * f[O + k] * h;
+                out[O + j] = acc;
+            }
+        }
+    } else {
+        // Standard orientation A[r][c] = delta_rc - h * J_rc, J_rc = Jt[c][r].
+        double A[n * n], x[n];
+#pragma unroll
+        for (int r = 0; r < n; r++)
+#pragma unroll
+            for (int cc = 0; cc < n; cc++)
+                A[r * n + cc] = (r == cc ? 1.0 : 0.0) - h.v * Jt[(O + cc) * N + O + r].v;
+#pragma unroll
+        for (int e = 0; e < n; e++) x[e] = f[O + e].v;
+        lu_solve_block<n, TRI>(A, x);
+#pragma unroll
+        for (int e = 0; e < n; e++) {
+            hi = max(hi, mag_hi(x[e]));
+            out[O + e] = y[O + e].v + h.v * x[e];
+        }
+    }
+    if (SOLVER == WIND_SOLVER_GJE_F64) {
+#pragma unroll
+        for (int e = 0; e < n; e++) hi = max(hi, mag_hi(out[O + e].v));
+    }
+}
+
+// One SIE or explicit-Euler substep of length h, in place on y: the FP64
+// solvers by the network's diagonal blocks.
+template <class Net, int METHOD, int CTRL, int SOLVER>
+__device__ __forceinline__ void lane_substep(const double (&c)[Net::NC], xd h, xd (&y)[Net::N]) {
+    if constexpr (METHOD == WIND_METHOD_RK2 || SOLVER == WIND_SOLVER_MIXED) {
+        lane_substep_full<Net, METHOD, CTRL, SOLVER>(c, h, y);
+    } else {
+        constexpr int N = Net::N;
+        static_assert(Net::B0 + Net::B1 == N, "blocks cover the network");
+        xd f[N], Jt[N * N], out[N];
+        Net::rhs(c, y, f);
+#pragma unroll
+        for (int e = 0; e < N * N; e++) Jt[e] = 0.0;
+        Net::jac(c, y, Jt);
+        int hi = 0;
+        lane_block_step<Net, CTRL, SOLVER, 0, Net::B0, false>(Jt, f, h, y, out, hi);
+        if constexpr (Net::B1 > 0)
+            lane_block_step<Net, CTRL, SOLVER, Net::B0, Net::B1, Net::TRI1>(Jt, f, h, y, out, hi);
+        if (hi >= HI_INF) {
+            double cs[Net::NC], ys[N];
+#pragma unroll
+            for (int k = 0; k < Net::NC; k++) cs[k] = c[k];
+#pragma unroll
+            for (int e = 0; e < N; e++) ys[e] = y[e].v;
+            lane_substep_redo<Net, CTRL, SOLVER>(cs, h.v, ys);
+#pragma unroll
+            for (int e = 0; e < N; e++) out[e] = ys[e];
+        }
+#pragma unroll
+        for (int e = 0; e < N; e++) y[e] = out[e];
+    }
 }
 
 // take_step (sie_gold.c:38-51) / innerstep (kernel.cu:69-91): nsub substeps
@@ -264,19 +379,28 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
             if (__all_sync(FULL, drained)) break;
             continue;
         }
-        // 2. assignment and state fetch
+        // 2. assignment and state fetch.  While every lane owns a system each
+        // works on its own at level 0: nothing to fetch.
+        const bool full = owners == FULL;
         const int nact = __popc(owners);
-        const int j = lane % nact;
-        const int r = lane / nact;
-        const int src = __fns(owners, 0, j + 1);
-        const int64_t s_j = __shfl_sync(FULL, s_own, src);
-        const double t_j = __shfl_sync(FULL, t_own, src);
-        const double h_j = __shfl_sync(FULL, h_own, src);
-        const int u_j = __shfl_sync(FULL, u_own, src);
-        const int64_t a_j = __shfl_sync(FULL, a_own, src);
+        int r = 0;
+        int64_t s_j = s_own, a_j = a_own;
+        double t_j = t_own, h_j = h_own;
+        int u_j = u_own;
         xd y[N];
 #pragma unroll
-        for (int i = 0; i < N; i++) y[i] = __shfl_sync(FULL, y_own[i], src);
+        for (int i = 0; i < N; i++) y[i] = y_own[i];
+        if (!full) {
+            r = lane / nact;
+            const int src = __fns(owners, 0, lane - r * nact + 1);
+            s_j = __shfl_sync(FULL, s_own, src);
+            t_j = __shfl_sync(FULL, t_own, src);
+            h_j = __shfl_sync(FULL, h_own, src);
+            u_j = __shfl_sync(FULL, u_own, src);
+            a_j = __shfl_sync(FULL, a_own, src);
+#pragma unroll
+            for (int i = 0; i < N; i++) y[i] = __shfl_sync(FULL, y_own[i], src);
+        }
         if (s_j != s_work) {
             s_work = s_j;
 #pragma unroll
@@ -300,12 +424,13 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
             for (int i = 0; i < N; i++) err |= elem_error<METHOD, CTRL>(y1[i], y2[i], p.atol, p.rtol);
         }
         const bool acc = valid && (!err || lvl == CAP);
-        const unsigned bal = __ballot_sync(FULL, acc);
         // 4. owners apply their team's outcome
         int take = lane;   // lane whose attempt this owner adopts (self = none)
-        int done = 0;      // attempts consumed this round
-        bool accepted = false;
-        if (has) {
+        int done = 1;      // attempts consumed this round
+        bool accepted = acc;
+        const unsigned bal = full ? 0u : __ballot_sync(FULL, acc);
+        if (!full && has) {
+            accepted = false;
             const int jo = __popc(owners & ((1u << lane) - 1u));
             const unsigned tm = team_mask_of(jo, nact, wmax);
             const int tsz = __popc(tm);
@@ -325,9 +450,12 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
 #pragma unroll
         for (int i = 0; i < N; i++)
             ytake[i] = (METHOD == WIND_METHOD_RK2) ? (xd(2.0) * y2[i] - y1[i]).v : y2[i].v;
-        const double htake = __shfl_sync(FULL, hl, take);
+        double htake = hl;
+        if (!full) {
+            htake = __shfl_sync(FULL, hl, take);
 #pragma unroll
-        for (int i = 0; i < N; i++) ytake[i] = __shfl_sync(FULL, ytake[i], take);
+            for (int i = 0; i < N; i++) ytake[i] = __shfl_sync(FULL, ytake[i], take);
+        }
         if (has) {
             a_own += done;
             if (accepted) {

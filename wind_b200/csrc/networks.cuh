@@ -7,6 +7,9 @@
 //                  writing only the nonzeros into a zero-filled J.
 // Builtin networks have a compile-time N so their state lives in registers.
 // Expression order follows the reference bodies exactly (bit-exact parity).
+// B0, B1: sizes of the Jacobian's diagonal blocks (B1 = 0: one block);
+// TRI1: the second block is tridiagonal.  The register solvers work block by
+// block (solvers_reg.cuh).
 #pragma once
 
 #include "common.cuh"
@@ -17,6 +20,8 @@ namespace wind {
 struct NetNR {
     static constexpr int N = 2;
     static constexpr int NC = 4;
+    static constexpr int B0 = 2, B1 = 0;
+    static constexpr bool TRI1 = false;
     template <class C, class Y, class F>
     __device__ __forceinline__ static void rhs(const C& c, const Y& y, F& f) {
         f[0] = xd(c[0]) * y[0] + xd(c[1]) * y[1];
@@ -35,6 +40,8 @@ struct NetNR {
 struct NetTrig {
     static constexpr int N = 2;
     static constexpr int NC = 2;
+    static constexpr int B0 = 2, B1 = 0;
+    static constexpr bool TRI1 = false;
     template <class C, class Y, class F>
     __device__ __forceinline__ static void rhs(const C& c, const Y& y, F& f) {
         f[0] = -y[0] + xd(c[1]) * y[1];
@@ -58,6 +65,8 @@ struct NetTrig {
 struct NetKatz96 {
     static constexpr int N = 5;
     static constexpr int NC = 10;
+    static constexpr int B0 = 2, B1 = 3;  // hydrogen {0, 1}, helium {2, 3, 4}
+    static constexpr bool TRI1 = true;
     template <class Y>
     __device__ __forceinline__ static xd ne_of(const Y& y) {
         return y[1] + y[3] + y[4] * 2.0;
@@ -115,6 +124,8 @@ struct NetKatz96 {
 struct NetKatz96Tile {
     static constexpr int N = 5;
     static constexpr int NC = 11;
+    static constexpr int B0 = 2, B1 = 3;  // hydrogen {0, 1}, helium {2, 3, 4}
+    static constexpr bool TRI1 = true;
     template <class C, class Y, class F>
     __device__ __forceinline__ static void rhs(const C& cc, const Y& y, F& f) {
         NetKatz96::rhs_ne(cc, xd(cc[10]), y, f);

@@ -126,4 +126,117 @@ __device__ __forceinline__ void lu_solve_reg(const T (&A)[N * N], const T (&rinv
     for (int i = 0; i < N; i++) b[i] = z[i];
 }
 
+// ---------------------------------------------------------------------------
+// Block forms.  The compiled networks' Jacobians are block diagonal (Katz96:
+// hydrogen 2x2, helium 3x3 tridiagonal), and an off-block entry of the
+// full-width eliminations above is an exact zero: a row operation with a zero
+// multiplier, a quotient 0/s or a product with a zero leaves every in-block
+// value as it is while nothing is infinite or NaN.  The block forms do the
+// in-block operations only, in the same order, so their results are the
+// full-width ones bit for bit (a zero's sign aside) whenever `max_hi` of the
+// values named below stays under HI_INF; otherwise the caller repeats the
+// substep full width.  A Katz96 substep then takes 12 divisions and 22
+// multiplications and subtractions in the Gauss-Jordan inverse instead of 50
+// and 1000, and one pivot comparison per column in the LU.
+constexpr int HI_INF = 0x7ff00000;
+__device__ __forceinline__ int mag_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// The reference's Gauss-Jordan inverse of one n x n block (reference
+// orientation).  Columns of M left of the pivot and columns of Inv right of it
+// are still zeros in the downward pass, and M's rows are unit rows by the time
+// the upward pass uses them.  `hi`: largest high word over the pivots.
+template <int n, bool TRI>
+__device__ __forceinline__ void gje_invert_block(xd (&M)[n * n], xd (&Inv)[n * n], int& hi) {
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        const xd s = M[i * n + i];
+        hi = max(hi, mag_hi(s.v));
+#pragma unroll
+        for (int t = i + 1; t < n; t++)
+            if (!TRI || t == i + 1) M[i * n + t] /= s;
+#pragma unroll
+        for (int t = 0; t < i; t++) Inv[i * n + t] /= s;
+        Inv[i * n + i] = xd(1.0) / s;
+#pragma unroll
+        for (int k = i + 1; k < n; k++) {
+            if (TRI && k > i + 1) continue;
+            const xd f = M[k * n + i];
+#pragma unroll
+            for (int t = i + 1; t < n; t++)
+                if (!TRI || t == i + 1) M[k * n + t] -= f * M[i * n + t];
+#pragma unroll
+            for (int t = 0; t <= i; t++) {
+                // Inv[k][t] is zero until the first row that reaches it
+                const bool first = TRI || t == i;
+                Inv[k * n + t] = first ? -(f * Inv[i * n + t]) : Inv[k * n + t] - f * Inv[i * n + t];
+            }
+        }
+    }
+#pragma unroll
+    for (int b = n - 1; b > 0; b--) {
+#pragma unroll
+        for (int k = b - 1; k >= 0; k--) {
+            if (TRI && k < b - 1) continue;
+            const xd f = M[k * n + b];
+#pragma unroll
+            for (int t = 0; t < n; t++) {
+                // right of the diagonal Inv[k][t] is zero until the first
+                // pivot row that reaches it
+                const bool first = t > k && (TRI || b == n - 1);
+                Inv[k * n + t] = first ? -(f * Inv[b * n + t]) : Inv[k * n + t] - f * Inv[b * n + t];
+            }
+        }
+    }
+}
+
+// Partial-pivot LU solve of one block, A x = b (x in place of b): the pivots,
+// multipliers and sums of lu_factor_reg / lu_solve_reg.  In a tridiagonal
+// block only the next row holds a nonzero below the pivot.
+template <int n, bool TRI>
+__device__ __forceinline__ void lu_solve_block(double (&A)[n * n], double (&b)[n]) {
+    double rinv[n];
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+        int p = i;
+        double best = fabs(A[i * n + i]);
+#pragma unroll
+        for (int k = i + 1; k < n; k++) {
+            if (TRI && k > i + 1) continue;
+            const double v = fabs(A[k * n + i]);
+            if (v > best) { best = v; p = k; }
+        }
+#pragma unroll
+        for (int k = i + 1; k < n; k++) {
+            if (TRI && k > i + 1) continue;
+            const bool sw = (p == k);
+#pragma unroll
+            for (int t = i; t < n; t++) {
+                const double u = A[i * n + t], w = A[k * n + t];
+                A[i * n + t] = sw ? w : u;
+                A[k * n + t] = sw ? u : w;
+            }
+            const double u = b[i], w = b[k];
+            b[i] = sw ? w : u;
+            b[k] = sw ? u : w;
+        }
+        const double r = nr_rcp(A[i * n + i]);
+        rinv[i] = r;
+#pragma unroll
+        for (int k = i + 1; k < n; k++) {
+            if (TRI && k > i + 1) continue;
+            const double l = A[k * n + i] * r;
+#pragma unroll
+            for (int t = i + 1; t < n; t++) A[k * n + t] = fma(-l, A[i * n + t], A[k * n + t]);
+            b[k] = fma(-l, b[i], b[k]);
+        }
+    }
+#pragma unroll
+    for (int i = n - 1; i >= 0; i--) {
+        double acc = b[i];
+#pragma unroll
+        for (int t = i + 1; t < n; t++) acc = fma(-A[i * n + t], b[t], acc);
+        b[i] = acc * rinv[i];
+    }
+}
+
 }  // namespace wind
