@@ -35,6 +35,7 @@ static MixedFn mixed_fn(int method, int ctrl, int solver) {
 
 static int nmax_of(int n) { return n <= 8 ? 8 : (n <= 16 ? 16 : 32); }
 bool team_admitted(int n, int R, bool lin, bool lists, int teams, size_t budget);
+bool warp_admitted(int n, int R, bool lin, int solver, int threads, size_t budget);
 
 // Launch all mass-action groups `ps` (kernel parameters with their counters
 // already set) in one kernel on `stream`.
@@ -58,13 +59,20 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
             const bool reg = o.method == WIND_METHOD_SIE && gs != WIND_SOLVER_GJE_F64;
             const bool plin = p.linear != nullptr;
             if (reg) {
-                smem = std::max(smem, (size_t)(MIXED_THREADS / nm) * WarpLayout(nm, p.n_react, plin, gs).bytes);
+                if (!warp_admitted(p.n_eq, p.n_react, plin, gs, MIXED_THREADS, (size_t)cap))
+                    return WIND_ERR_UNSUPPORTED;
+                size_t bytes = (size_t)(MIXED_THREADS / nm) * WarpLayout(nm, p.n_react, plin, gs).bytes;
+                if (gs == WIND_SOLVER_LU_F64) {
+                    const LuLayout lay(nm, p.n_eq, p.n_react, plin);
+                    bytes = (size_t)mixed_teams(nm, lay.bytes, cap) * lay.bytes;
+                }
+                smem = std::max(smem, bytes);
             } else {
                 if (!team_admitted(p.n_eq, p.n_react, plin, o.method == WIND_METHOD_RK2, MIXED_THREADS / nm,
                                    (size_t)cap))
                     return WIND_ERR_UNSUPPORTED;
                 const TeamLayout lay(nm, p.n_react, plin, o.method == WIND_METHOD_SIE);
-                smem = std::max(smem, (size_t)mixed_teams(nm, lay, cap) * lay.bytes);
+                smem = std::max(smem, (size_t)mixed_teams(nm, lay.bytes, cap) * lay.bytes);
             }
         }
     }

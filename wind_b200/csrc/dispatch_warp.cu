@@ -1,5 +1,5 @@
-// dispatch_warp.cu -- launch of the register-resident team kernels (mass
-// action, N <= 32, SIE with the LU_F64 or MIXED solver).
+// dispatch_warp.cu -- launch of the register-resident MIXED team kernels (mass
+// action, N <= 32, SIE); LU_F64 goes to dispatch_lu.cu.
 #include <mutex>
 #include <vector>
 
@@ -10,16 +10,9 @@ namespace wind {
 
 using WarpFn = void (*)(KParams);
 
-template <int NMAX, int CTRL>
-static WarpFn warp_by_solver(int solver) {
-    return solver == WIND_SOLVER_MIXED ? k_warp<NMAX, CTRL, WIND_SOLVER_MIXED>
-                                       : k_warp<NMAX, CTRL, WIND_SOLVER_LU_F64>;
-}
-
 template <int NMAX>
-static WarpFn warp_fn(int ctrl, int solver) {
-    return ctrl == WIND_CTRL_GOLD ? warp_by_solver<NMAX, WIND_CTRL_GOLD>(solver)
-                                  : warp_by_solver<NMAX, WIND_CTRL_DEVICE>(solver);
+static WarpFn warp_fn(int ctrl) {
+    return ctrl == WIND_CTRL_GOLD ? k_warp<NMAX, WIND_CTRL_GOLD> : k_warp<NMAX, WIND_CTRL_DEVICE>;
 }
 
 int warp_nmax(int n) { return n <= 8 ? 8 : (n <= 16 ? 16 : 32); }
@@ -48,11 +41,20 @@ static int warp_blocks_per_sm(WarpFn fn, int threads, size_t smem) {
     return nb;
 }
 
+// Whether N species and R reactions are accepted: what fits a full block of
+// these kernels' slices, for the LU kernels too, whose own slices differ.
+bool warp_admitted(int n, int R, bool lin, int solver, int threads, size_t budget) {
+    return warp_smem_bytes(n, R, lin, solver, threads) <= budget;
+}
+
+wind_status launch_lu(const wind_options& o, const KParams& p, cudaStream_t stream);
+
 wind_status launch_warp(const wind_options& o, const KParams& p, cudaStream_t stream) {
+    if (o.solver == WIND_SOLVER_LU_F64) return launch_lu(o, p, stream);
     const int nmax = warp_nmax(p.n_eq);
-    WarpFn fn = nmax == 8 ? warp_fn<8>(o.controller, o.solver)
-              : nmax == 16 ? warp_fn<16>(o.controller, o.solver)
-                           : warp_fn<32>(o.controller, o.solver);
+    WarpFn fn = nmax == 8 ? warp_fn<8>(o.controller)
+              : nmax == 16 ? warp_fn<16>(o.controller)
+                           : warp_fn<32>(o.controller);
     const int threads = WARP_THREADS;
     const size_t smem = warp_smem_bytes(p.n_eq, p.n_react, p.linear != nullptr, o.solver, threads);
     if (smem > 227 * 1024) return WIND_ERR_UNSUPPORTED;

@@ -12,6 +12,7 @@
 #pragma once
 
 #include "cta_kernel.cuh"
+#include "lu_kernel.cuh"
 #include "team_kernel.cuh"
 #include "warp_kernel.cuh"
 
@@ -19,17 +20,27 @@ namespace wind {
 
 constexpr int MIXED_THREADS = CTA_THREADS;
 
-// Teams of a block that run a group of the team kernel: all that the lanes
-// hold, or as many as the shared-memory budget does.
-__host__ __device__ inline int mixed_teams(int nmax, const TeamLayout& lay, int smem_cap) {
-    const int full = MIXED_THREADS / nmax, fit = smem_cap / lay.bytes;
+// Teams of a block that run a group of the team or LU kernel: all that the
+// lanes hold, or as many as the shared-memory budget does.
+__host__ __device__ inline int mixed_teams(int nmax, int team_bytes, int smem_cap) {
+    const int full = MIXED_THREADS / nmax, fit = smem_cap / team_bytes;
     return fit < full ? fit : full;
 }
 
 template <int NMAX, int METHOD, int CTRL>
 __device__ __forceinline__ void mixed_team_run(const KParams& p, unsigned char* smem_raw, int smem_cap) {
     const TeamLayout lay(NMAX, p.n_react, p.linear != nullptr, METHOD == WIND_METHOD_SIE);
-    team_run<NMAX, METHOD, CTRL>(p, smem_raw, mixed_teams(NMAX, lay, smem_cap), 32 / NMAX);
+    team_run<NMAX, METHOD, CTRL>(p, smem_raw, mixed_teams(NMAX, lay.bytes, smem_cap), 32 / NMAX);
+}
+
+template <int NMAX, int CTRL, int SOLVER>
+__device__ __forceinline__ void mixed_warp_run(const KParams& p, unsigned char* smem_raw, int smem_cap) {
+    if constexpr (SOLVER == WIND_SOLVER_LU_F64) {
+        const LuLayout lay(NMAX, p.n_eq, p.n_react, p.linear != nullptr);
+        lu_run<NMAX, NMAX, true, CTRL>(p, smem_raw, mixed_teams(NMAX, lay.bytes, smem_cap), 32 / NMAX);
+    } else {
+        warp_run<NMAX, CTRL>(p, smem_raw);
+    }
 }
 
 // Two blocks per SM (128 registers) for the LU and mixed solvers, whose team
@@ -48,9 +59,9 @@ __global__ void __launch_bounds__(MIXED_THREADS, SOLVER == WIND_SOLVER_GJE_F64 ?
             constexpr bool REG = METHOD == WIND_METHOD_SIE && SMALL != WIND_SOLVER_GJE_F64;
             if (p.n_eq > 32) cta_run<METHOD, CTRL, SOLVER, false>(p, smem_raw, gscratch, gstride, smem_cap);
             else if constexpr (REG) {
-                if (p.n_eq > 16) warp_run<32, CTRL, SMALL>(p, smem_raw);
-                else if (p.n_eq > 8) warp_run<16, CTRL, SMALL>(p, smem_raw);
-                else warp_run<8, CTRL, SMALL>(p, smem_raw);
+                if (p.n_eq > 16) mixed_warp_run<32, CTRL, SMALL>(p, smem_raw, smem_cap);
+                else if (p.n_eq > 8) mixed_warp_run<16, CTRL, SMALL>(p, smem_raw, smem_cap);
+                else mixed_warp_run<8, CTRL, SMALL>(p, smem_raw, smem_cap);
             } else {
                 if (p.n_eq > 16) mixed_team_run<32, METHOD, CTRL>(p, smem_raw, smem_cap);
                 else if (p.n_eq > 8) mixed_team_run<16, METHOD, CTRL>(p, smem_raw, smem_cap);

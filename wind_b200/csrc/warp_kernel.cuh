@@ -1,5 +1,6 @@
-// warp_kernel.cuh -- register-resident team-per-system SIE for runtime
-// mass-action networks with N <= 32 (optionally with a dense linear term).
+// warp_kernel.cuh -- register-resident team-per-system SIE with the MIXED solver
+// for runtime mass-action networks with N <= 32 (optionally with a dense linear
+// term), and the row-per-lane pieces the semi-implicit midpoint kernel shares.
 //
 // A team is NMAX lanes of one warp (NMAX = 8, 16 or 32); a 128-thread block
 // holds 128/NMAX teams, each with its own shared-memory slice.  Lane l owns
@@ -11,29 +12,21 @@
 // elimination steps are unrolled, so a step costs one reduction for the
 // pivot, one row broadcast and NMAX fused multiply-adds per lane.
 //
-// Solvers (SIE only; RK2 and the reference Gauss-Jordan stay in the team
-// kernel):
-//  LU_F64  the plain FP64 path: I - hJ built at every substep, LU with
-//          partial pivoting (pivot = one warp reduction over a packed
-//          |a|/lane key, rows never move), right-hand side eliminated with the
-//          factorisation, column-oriented back substitution;
-//  MIXED   FP32 Gauss-Jordan inverse of I - hJ with partial pivoting, computed
-//          ONCE per step-doubling attempt at the half-step size and the
-//          attempt's state, and used as the approximate inverse of every solve
-//          of the attempt (both half steps, and the next attempt's full step
-//          after a rejection, whose size is that half-step size) inside an
-//          FP64 iterative refinement: r = f - (x - h J x) in FP64 from the
-//          network itself at the substep's own state, x += M r, until the
-//          predicted error is below 2^-33 |x|.  A refinement that stalls is
-//          restarted with a fresh inverse of the substep's own matrix; if that
-//          one does not refine either (I - hJ too ill-conditioned for FP32),
-//          the substep is solved by the plain FP64 LU, the system is flagged
-//          WIND_SYS_REFINE_FALLBACK, and its substeps of that size and larger
-//          go straight to the FP64 LU from then on.
+// MIXED: FP32 Gauss-Jordan inverse of I - hJ with partial pivoting, computed
+// ONCE per step-doubling attempt at the half-step size and the attempt's state,
+// and used as the approximate inverse of every solve of the attempt (both half
+// steps, and the next attempt's full step after a rejection, whose size is that
+// half-step size) inside an FP64 iterative refinement: r = f - (x - h J x) in
+// FP64 from the network itself at the substep's own state, x += M r, until the
+// predicted error is below 2^-33 |x|.  A refinement that stalls is restarted
+// with a fresh inverse of the substep's own matrix; if that one does not refine
+// either (I - hJ too ill-conditioned for FP32), the substep is solved by a
+// partial-pivot FP64 LU, the system is flagged WIND_SYS_REFINE_FALLBACK, and its
+// substeps of that size and larger go straight to the FP64 LU from then on.
 // The step sizes, substep sequence, error test and accept/reject decisions
 // are the reference controller's (cuda/common/kernel.cu:191-296 DEVICE,
 // cuda/c_baseline/common/common_gold.c:48-153 GOLD); only the linear solve
-// differs.
+// differs.  (LU_F64: lu_kernel.cuh.)
 #pragma once
 
 #include <type_traits>
@@ -286,34 +279,6 @@ __device__ __forceinline__ double warp_lu_solve(const WarpCtx<NMAX, double>& c, 
     return xl;
 }
 
-// I - hJ from the scatter rows, solved by the FP64 LU, as one out-of-line
-// body: the three solves of an attempt share its instructions (inlined, each
-// was its own copy of the unrolled elimination, and the kernel stalled on
-// instruction fetch).
-// The context's fields travel as scalars, so the call passes them in
-// registers instead of through a stack copy of the whole context.
-template <int NMAX>
-__device__ __noinline__ double warp_lu_solve_at(unsigned mask, int l, int leader, int N,
-                                                const float* LT, double* rows, double* pb, int* piv,
-                                                double h, double b) {
-    WarpCtx<NMAX, double> c;
-    c.mask = mask;
-    c.l = l;
-    c.leader = leader;
-    c.N = N;
-    c.LT = LT;
-    c.rows = rows;
-    c.pb = pb;
-    c.piv = piv;
-    double a[NMAX];
-    warp_load_matrix(c, h, a);
-    return warp_lu_solve(c, a, b);
-}
-template <int NMAX>
-__device__ __forceinline__ double warp_lu_solve_at(const WarpCtx<NMAX, double>& c, double h, double b) {
-    return warp_lu_solve_at<NMAX>(c.mask, c.l, c.leader, c.N, c.LT, c.rows, c.pb, c.piv, h, b);
-}
-
 // ---- FP32 Gauss-Jordan inverse --------------------------------------------
 // In-place inversion of A (row l in a[]) with partial pivoting and no row
 // exchanges: after step k the pivot lane's row expresses unknown k.  The
@@ -535,12 +500,12 @@ __device__ __forceinline__ bool warp_stage_system(const WarpCtx<NMAX, T>& c, con
     return bad_idx;
 }
 
-template <int NMAX, int CTRL, int SOLVER>
+template <int NMAX, int CTRL>
 __device__ __forceinline__ void warp_run(const KParams& p, unsigned char* smem_raw) {
-    using T = typename std::conditional<SOLVER == WIND_SOLVER_MIXED, float, double>::type;
+    using T = float;
     constexpr int CAP = Cap<WIND_METHOD_SIE, CTRL>::value;
     const bool lin = p.linear != nullptr;
-    const WarpLayout lay(NMAX, p.n_react, lin, SOLVER);
+    const WarpLayout lay(NMAX, p.n_react, lin, WIND_SOLVER_MIXED);
     const int team = threadIdx.x / NMAX;
     const int lane = threadIdx.x & 31;
     WarpCtx<NMAX, T> c;
@@ -602,24 +567,21 @@ __device__ __forceinline__ void warp_run(const KParams& p, unsigned char* smem_r
         // state in vb): FP32 inverse and FP64 refinement, or the FP64 LU.
         auto mixed_fresh = [&](double hh, double ff, bool save) -> double {
             double xx = 0.0;
-            if constexpr (SOLVER == WIND_SOLVER_MIXED) {
-                if (hh < h_fp64) {
-                    warp_load_matrix(c, hh, a);
-                    mystep = warp_gj_invert(c, a);
-                    if (warp_refine(c, a, mystep, hh, ff, xx, WARP_MIX_MAXIT2, 0.25) == REFINE_OK) {
-                        if (save) {
-                            warp_save_inverse(c, a);
-                            svstep = mystep;
-                            inv_ok = true;
-                        }
-                        return xx;
+            if (hh < h_fp64) {
+                warp_load_matrix(c, hh, a);
+                mystep = warp_gj_invert(c, a);
+                if (warp_refine(c, a, mystep, hh, ff, xx, WARP_MIX_MAXIT2, 0.25) == REFINE_OK) {
+                    if (save) {
+                        warp_save_inverse(c, a);
+                        svstep = mystep;
+                        inv_ok = true;
                     }
-                    h_fp64 = hh;
+                    return xx;
                 }
-                st |= WIND_SYS_REFINE_FALLBACK;
-                xx = warp_fp64_fallback(c, hh, ff);
+                h_fp64 = hh;
             }
-            return xx;
+            st |= WIND_SYS_REFINE_FALLBACK;
+            return warp_fp64_fallback(c, hh, ff);
         };
         while (!bad_idx && tnow < tend) {
             if (attempts >= p.max_attempts) { st |= WIND_SYS_MAX_ATTEMPTS; break; }
@@ -640,54 +602,38 @@ __device__ __forceinline__ void warp_run(const KParams& p, unsigned char* smem_r
             __syncwarp(c.mask);
             if (!fy_ok) { fy = warp_rhs(c); fy_ok = true; }
             if (!jy_ok) { warp_jma_row(c); jy_ok = true; }
-            double y1, vh;
-            if constexpr (SOLVER == WIND_SOLVER_MIXED) {
-                double x;
-                // full step: the previous attempt's half-step inverse is
-                // the inverse of this matrix (same state, same size) when y
-                // is unchanged; else a fresh one
-                if (hf < h_fp64 && inv_ok) {
-                    warp_load_inverse(c, a);
-                    mystep = svstep;
-                    if (warp_refine(c, a, mystep, hf, fy, x, WARP_MIX_MAXIT, 0.5) != REFINE_OK)
-                        x = mixed_fresh(hf, fy, false);
-                } else {
+            double x;
+            // full step: the previous attempt's half-step inverse is the
+            // inverse of this matrix (same state, same size) when y is
+            // unchanged; else a fresh one
+            if (hf < h_fp64 && inv_ok) {
+                warp_load_inverse(c, a);
+                mystep = svstep;
+                if (warp_refine(c, a, mystep, hf, fy, x, WARP_MIX_MAXIT, 0.5) != REFINE_OK)
                     x = mixed_fresh(hf, fy, false);
-                }
-                y1 = y + hf * x;
-                // first half step: a fresh inverse, saved for the next attempt
-                inv_ok = false;
-                x = mixed_fresh(h1, fy, true);
-                vh = y + h1 * x;
             } else {
-                y1 = y + hf * warp_lu_solve_at(c, hf, fy);
-                __syncwarp(c.mask);
-                vh = y + h1 * warp_lu_solve_at(c, h1, fy);
+                x = mixed_fresh(hf, fy, false);
             }
+            const double y1 = y + hf * x;
+            // first half step: a fresh inverse, saved for the next attempt
+            inv_ok = false;
+            x = mixed_fresh(h1, fy, true);
+            const double vh = y + h1 * x;
             // ---- second half step from vh
             __syncwarp(c.mask);
             if (l < N) c.vb[l] = vh;
             __syncwarp(c.mask);
             const double f2 = warp_rhs(c);
-            double y2;
-            if constexpr (SOLVER == WIND_SOLVER_MIXED) {
-                double x;
-                // the half-step inverse again, if it still contracts well at
-                // vh (small steps); else an inverse of this substep's own
-                // matrix (the scatter rows then hold J(vh), not J(y))
-                if (!inv_ok || h2 >= h_fp64 ||
-                    warp_refine(c, a, mystep, h2, f2, x, WARP_MIX_MAXIT, 0.0625) != REFINE_OK) {
-                    warp_jma_row(c);
-                    jy_ok = false;
-                    x = mixed_fresh(h2, f2, false);
-                }
-                y2 = vh + h2 * x;
-            } else {
+            // the half-step inverse again, if it still contracts well at vh
+            // (small steps); else an inverse of this substep's own matrix (the
+            // scatter rows then hold J(vh), not J(y))
+            if (!inv_ok || h2 >= h_fp64 ||
+                warp_refine(c, a, mystep, h2, f2, x, WARP_MIX_MAXIT, 0.0625) != REFINE_OK) {
                 warp_jma_row(c);
                 jy_ok = false;
-                __syncwarp(c.mask);
-                y2 = vh + h2 * warp_lu_solve_at(c, h2, f2);
+                x = mixed_fresh(h2, f2, false);
             }
+            const double y2 = vh + h2 * x;
             bool err = false;
             if (l < N) err = elem_error<WIND_METHOD_SIE, CTRL>(xd(y1), xd(y2), p.atol, p.rtol);
             err = __any_sync(c.mask, err);
@@ -718,10 +664,10 @@ __device__ __forceinline__ void warp_run(const KParams& p, unsigned char* smem_r
     }
 }
 
-template <int NMAX, int CTRL, int SOLVER>
+template <int NMAX, int CTRL>
 __global__ void __launch_bounds__(WARP_THREADS, 4) k_warp(const KParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    warp_run<NMAX, CTRL, SOLVER>(p, smem_raw);
+    warp_run<NMAX, CTRL>(p, smem_raw);
 }
 
 }  // namespace wind
