@@ -98,8 +98,13 @@ wind_status launch_integrate(const wind_options& o_in, const KParams& p, cudaStr
     if (pst != WIND_OK) return pst;
     if (pl.gstride == 0) return launch_cta(pl, p, stream, nullptr);
     double* scratch = nullptr;
-    if (cudaMallocAsync((void**)&scratch, (size_t)pl.grid * pl.gstride * sizeof(double), stream) != cudaSuccess)
-        return WIND_ERR_NOMEM;
+    if (cudaMallocAsync((void**)&scratch, (size_t)pl.grid * pl.gstride * sizeof(double), stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        pl.gstride = pl.need;
+        if (pl.need == 0) return launch_cta(pl, p, stream, nullptr);
+        if (cudaMallocAsync((void**)&scratch, (size_t)pl.grid * pl.gstride * sizeof(double), stream) != cudaSuccess)
+            return WIND_ERR_NOMEM;
+    }
     const wind_status st = launch_cta(pl, p, stream, scratch);
     cudaFreeAsync(scratch, stream);
     return st;

@@ -46,11 +46,12 @@ wind_status launch_lane(const wind_options& o, const KParams& p, cudaStream_t st
 // Tiled builtin network (n_eq = Ntile x base_n, 1 < Ntile <= WIND_MAX_TILES).
 wind_status launch_tile(const wind_options& o, const KParams& p, int base_n, cudaStream_t stream);
 // A CTA-kernel launch: kernel, shared-memory budget and size, grid, and
-// the per-block global scratch (doubles; 0 = none).
+// the per-block global scratch (doubles; 0 = none): what the launch asks for and
+// what it cannot do without.
 struct CtaPlan {
     const void* fn;
-    int smem_cap, smem_bytes, grid;
-    size_t gstride;
+    int threads, smem_cap, smem_bytes, grid;
+    size_t gstride, need;
 };
 wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global, CtaPlan* out);
 wind_status launch_cta(const CtaPlan& pl, const KParams& p, cudaStream_t stream, double* scratch);

@@ -1,5 +1,6 @@
 // dispatch_cta.cu -- instantiations and launch of the CTA-per-system kernels
 // (mass action, 32 < N <= 256).
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -49,16 +50,17 @@ static int smem_half(CtaFn fn) {
     return (int)((per_sm / 2 - 1024 - (int)stat) & ~127);
 }
 
-static int cta_blocks_per_sm(CtaFn fn, size_t smem) {
+static int cta_blocks_per_sm(CtaFn fn, int threads, size_t smem) {
     static std::mutex mu;
-    static std::vector<std::pair<std::pair<const void*, size_t>, int>> cache;
+    static std::vector<std::pair<std::pair<const void*, size_t>, std::pair<int, int>>> cache;
     std::lock_guard<std::mutex> g(mu);
     for (auto& e : cache)
-        if (e.first.first == (const void*)fn && e.first.second == smem) return e.second;
+        if (e.first.first == (const void*)fn && e.first.second == smem && e.second.first == threads)
+            return e.second.second;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, CTA_THREADS, smem) != cudaSuccess) nb = 0;
-    cache.push_back({{(const void*)fn, smem}, nb});
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess) nb = 0;
+    cache.push_back({{(const void*)fn, smem}, {threads, nb}});
     return nb;
 }
 
@@ -77,12 +79,16 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
     const int solver = method_solver(o);
     const bool tc = o.method == WIND_METHOD_SIE && o.solver == WIND_SOLVER_MIXED_TC;
     CtaFn fn = cta_fn(o.method, o.controller, o.solver);
+    // up to 128 species: 128 threads (600 systems of 64 species: 71.9 ms, 72.6
+    // with 256).  Shared memory for four of those blocks per SM would push the
+    // reaction records out to L2: 113.6 ms.
+    const int threads = p.n_eq <= CTA_THREADS / 2 && !tc ? CTA_THREADS / 2 : CTA_THREADS;
     int caps[2] = {smem_optin(), 0};
     int ncap = 1;
     if (solver == WIND_SOLVER_MIXED && CtaMinBlocks<WIND_SOLVER_MIXED>::value >= 2) caps[ncap++] = smem_half(fn);
     // ranking: the matrix in shared memory first (a matrix in global memory
     // is read and written on every trailing update), then blocks per SM;
-    // ties keep the larger budget
+    // the batch can use; ties keep the larger budget
     bool found = false;
     CtaPlan best{};
     int best_score = 0;
@@ -93,15 +99,18 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
         // with it (the MMA operands are built from it every panel)
         if (tc && !lay.mat_in_smem) continue;
         if (!allow_global && lay.g_doubles > 0) continue;
-        const int nb = cta_blocks_per_sm(fn, lay.bytes);
-        const int score = nb + (lay.mat_in_smem ? 1000 : 0);
+        const int nb = cta_blocks_per_sm(fn, threads, lay.bytes);
+        const int used = (int)std::min<int64_t>(nb, (p.nsys + device_sm_count() - 1) / device_sm_count());
+        const int score = used + (lay.mat_in_smem ? 1000 : 0);
         if (nb < 1 || score <= best_score) continue;
         const int64_t resident = (int64_t)nb * device_sm_count();
         best.fn = (const void*)fn;
+        best.threads = threads;
         best.smem_cap = caps[i];
         best.smem_bytes = lay.bytes;
         best.grid = (int)(p.nsys < resident ? p.nsys : resident);
-        best.gstride = lay.g_doubles;
+        best.gstride = allow_global ? lay.slot_doubles() : lay.g_doubles;
+        best.need = lay.g_doubles;
         best_score = score;
         found = true;
     }
@@ -112,17 +121,17 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
 
 size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int solver) {
     const CtaLayout lay(n_eq, n_react, lin, solver, smem_optin());
-    return lay.g_doubles * sizeof(double);
+    return lay.slot_doubles() * sizeof(double);
 }
 
 wind_status launch_cta(const CtaPlan& pl, const KParams& p, cudaStream_t stream, double* scratch) {
-    if (pl.gstride && !scratch) return WIND_ERR_ARGUMENT;
+    if (pl.need && !scratch) return WIND_ERR_ARGUMENT;
     CtaFn fn = reinterpret_cast<CtaFn>(const_cast<void*>(pl.fn));
     // set for this launch every time (the occupancy cache may come from a
     // launch of the same kernel with another size)
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes) != cudaSuccess)
         return launch_status("k_cta shared-memory attribute");
-    fn<<<pl.grid, CTA_THREADS, pl.smem_bytes, stream>>>(p, pl.gstride ? scratch : nullptr, pl.gstride,
+    fn<<<pl.grid, pl.threads, pl.smem_bytes, stream>>>(p, pl.gstride ? scratch : nullptr, scratch ? pl.gstride : 0,
                                                         pl.smem_cap);
     g_launches++;
     return launch_status("k_cta launch");

@@ -46,14 +46,15 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cap -= 1024;
-    size_t smem = 0, gslot = 0;
+    size_t smem = 0, gslot = 0, gneed = 0;
     for (const KParams& p : ps) {
         // the solver each group runs (AUTO: MIXED above 32 species, LU_F64 below)
         const int gs = resolve_solver(solver, p.kind, p.n_eq);
         if (p.n_eq > 32) {
             const CtaLayout lay(p.n_eq, p.n_react, p.linear != nullptr, gs, cap);
             smem = std::max(smem, (size_t)lay.bytes);
-            gslot = std::max(gslot, lay.g_doubles);
+            gslot = std::max(gslot, lay.slot_doubles());
+            gneed = std::max(gneed, lay.g_doubles);
         } else {
             const int nm = nmax_of(p.n_eq);
             const bool reg = o.method == WIND_METHOD_SIE && gs != WIND_SOLVER_GJE_F64;
@@ -96,6 +97,12 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
     if (cudaMallocAsync((void**)&dparams, pbytes + obytes + 16, stream) != cudaSuccess) return WIND_ERR_NOMEM;
     double* gscratch = nullptr;
     if (gslot && cudaMallocAsync((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        gscratch = nullptr;
+        gslot = gneed;
+    }
+    if (gslot && !gscratch &&
+        cudaMallocAsync((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
         cudaFreeAsync(dparams, stream);
         return WIND_ERR_NOMEM;
     }
