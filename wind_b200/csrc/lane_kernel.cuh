@@ -292,10 +292,34 @@ __device__ __forceinline__ void lane_attempt(const double (&c)[Net::NC], double 
 // systems in the warp (owners), lane i works on owner (i mod a) at
 // refinement level (i div a): lanes are spread round-robin, so team sizes
 // differ by at most one and the lowest lane of a team carries level 0.
-__device__ __forceinline__ unsigned team_mask_of(int j, int nact, int wmax) {
-    unsigned m = 0u;
-    for (int k = j, r = 0; k < 32 && r < wmax; k += nact, r++) m |= 1u << k;
+
+// Bits 0, n, 2n, ... below 32.
+__device__ __forceinline__ unsigned every_nth(int n) {
+    unsigned m = 1u;
+    for (int s = n; s < 32; s <<= 1) m |= m << s;
     return m;
+}
+// Position of the n-th (from 0) set bit of m.
+__device__ __forceinline__ int nth_bit(unsigned m, int n) {
+    int pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const int c = __popc(m & ((1u << w) - 1u));
+        if (n >= c) {
+            n -= c;
+            m >>= w;
+            pos += w;
+        }
+    }
+    return pos;
+}
+// x halved n times (0 <= n <= 32): one exact multiplication while the result
+// stays normal.
+__device__ __forceinline__ double halved(double x, int n) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    if (e > 32) return x * __hiloint2double((1023 - n) << 20, 0);
+    for (int q = 0; q < n; q++) x /= 2.0;
+    return x;
 }
 
 // Persistent kernel.  Every lane owns at most one system (its state lives in
@@ -321,7 +345,6 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
     constexpr int NC = Net::NC;
     constexpr int CAP = Cap<METHOD, CTRL>::value;
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr int wmax = 32;
     const int lane = threadIdx.x & 31;
     const uint64_t t_start = p.timeout_ns ? global_ns() : 0;
     const double tend = p.tend;
@@ -337,6 +360,9 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
     // worker cache
     int64_t s_work = -1;
     double c[NC];
+    // the warp's assignment, kept while the owners stay the same lanes
+    unsigned owners_at = 0u, team = 0u;
+    int src = lane, r = 0;
 
     while (true) {
         // 1. refill: take new tickets while without a system
@@ -382,8 +408,13 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
         // 2. assignment and state fetch.  While every lane owns a system each
         // works on its own at level 0: nothing to fetch.
         const bool full = owners == FULL;
-        const int nact = __popc(owners);
-        int r = 0;
+        if (owners != owners_at) {
+            owners_at = owners;
+            const int nact = __popc(owners);
+            r = lane / nact;
+            src = nth_bit(owners, lane - r * nact);
+            team = every_nth(nact) << __popc(owners & ((1u << lane) - 1u));  // (owners')
+        }
         int64_t s_j = s_own, a_j = a_own;
         double t_j = t_own, h_j = h_own;
         int u_j = u_own;
@@ -391,8 +422,6 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
 #pragma unroll
         for (int i = 0; i < N; i++) y[i] = y_own[i];
         if (!full) {
-            r = lane / nact;
-            const int src = __fns(owners, 0, lane - r * nact + 1);
             s_j = __shfl_sync(FULL, s_own, src);
             t_j = __shfl_sync(FULL, t_own, src);
             h_j = __shfl_sync(FULL, h_own, src);
@@ -409,10 +438,9 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
         // 3. one attempt at level r: kernel.cu:195 / common_gold.c:79 clamp,
         //    then r halvings (kernel.cu:262 / common_gold.c:123)
         const double hw = fmin(tend - t_j, h_j);
-        double hl = hw;
-        for (int q = 0; q < r; q++) hl /= 2.0;
+        const double hl = halved(hw, r);
         const int lvl = u_j + r;
-        const bool valid = (r < wmax) && (lvl <= CAP) && (a_j + r < p.max_attempts);
+        const bool valid = (lvl <= CAP) && (a_j + r < p.max_attempts);
         xd y1[N], y2[N];
 #pragma unroll
         for (int i = 0; i < N; i++) { y1[i] = y[i]; y2[i] = y[i]; }
@@ -431,17 +459,14 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
         const unsigned bal = full ? 0u : __ballot_sync(FULL, acc);
         if (!full && has) {
             accepted = false;
-            const int jo = __popc(owners & ((1u << lane) - 1u));
-            const unsigned tm = team_mask_of(jo, nact, wmax);
-            const int tsz = __popc(tm);
-            const unsigned mine = bal & tm;
+            const unsigned mine = bal & team;
             if (mine) {
                 take = __ffs(mine) - 1;
-                done = take / nact + 1;
+                done = __popc(team & ((1u << take) - 1u)) + 1;
                 accepted = true;
             } else {
                 // every level of the team refined (the cap level would accept)
-                int lim = tsz;
+                int lim = __popc(team);
                 if (a_own + lim > p.max_attempts) lim = (int)(p.max_attempts - a_own);
                 done = lim;
             }
@@ -472,9 +497,7 @@ __global__ void __launch_bounds__(LANE_THREADS, LaneMinBlocks<SOLVER>::value) k_
                 }
             } else {
                 u_own += done;
-                double hh = fmin(tend - t_own, h_own);
-                for (int q = 0; q < done; q++) hh /= 2.0;
-                h_own = hh;
+                h_own = halved(fmin(tend - t_own, h_own), done);
             }
         }
     }
