@@ -90,6 +90,14 @@ inline bool device_ptr(const void* ptr) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Stream-ordered device memory from the library's own pool of the current device
+// (api.cu).  The device's default pool gives everything back at every
+// synchronisation, and a call after an idle moment then maps its memory again
+// (about 0.4 ms); this one keeps up to POOL_KEEP bytes.  Freed with
+// cudaFreeAsync; safe from any thread and on any stream.
+constexpr uint64_t POOL_KEEP = 64ull << 20;
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t stream);
+
 // One wind_integrate call: device copies of host inputs (when memory is
 // HOST), the counters block, and the kernel parameters.  Allocations are
 // stream-ordered (cudaMallocAsync / cudaFreeAsync) and released in release().
@@ -108,7 +116,7 @@ struct IntegrateCall {
     void* alloc(size_t bytes) {
         void* p = nullptr;
         if (bytes == 0) bytes = 16;
-        if (cudaMallocAsync(&p, bytes, stream) != cudaSuccess) { failed = true; return nullptr; }
+        if (pool_alloc(&p, bytes, stream) != cudaSuccess) { failed = true; return nullptr; }
         allocs[nalloc++] = p;
         return p;
     }

@@ -68,7 +68,7 @@ wind_status launch_batch(const wind_options& o, const wind_group* groups, int ng
     }
     if (ngroups == 0) return WIND_OK;
     unsigned long long* counters = nullptr;
-    if (cudaMallocAsync((void**)&counters, (size_t)ngroups * CNT_SLOTS * 8, stream) != cudaSuccess)
+    if (pool_alloc((void**)&counters, (size_t)ngroups * CNT_SLOTS * 8, stream) != cudaSuccess)
         return WIND_ERR_NOMEM;
     cudaMemsetAsync(counters, 0, (size_t)ngroups * CNT_SLOTS * 8, stream);
     std::vector<KParams> mass, builtin;

@@ -94,15 +94,15 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
     });
     const size_t pbytes = ps.size() * sizeof(KParams), obytes = order.size() * sizeof(int);
     unsigned char* dparams = nullptr;
-    if (cudaMallocAsync((void**)&dparams, pbytes + obytes + 16, stream) != cudaSuccess) return WIND_ERR_NOMEM;
+    if (pool_alloc((void**)&dparams, pbytes + obytes + 16, stream) != cudaSuccess) return WIND_ERR_NOMEM;
     double* gscratch = nullptr;
-    if (gslot && cudaMallocAsync((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
+    if (gslot && pool_alloc((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
         (void)cudaGetLastError();
         gscratch = nullptr;
         gslot = gneed;
     }
     if (gslot && !gscratch &&
-        cudaMallocAsync((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
+        pool_alloc((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
         cudaFreeAsync(dparams, stream);
         return WIND_ERR_NOMEM;
     }

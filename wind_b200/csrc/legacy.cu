@@ -34,6 +34,11 @@
 #error "WIND_LEGACY_METHOD must be WIND_METHOD_SIE or WIND_METHOD_RK2"
 #endif
 
+// libwind's integration of float32 host arrays (api.cu), in place on y.
+extern "C" int wind_integrate_f32(const wind_options* opt, int32_t kind, int32_t n_eq, int32_t n_const, double tnow,
+                                  double tend, int32_t n_integration_steps, const float* constants, float* y,
+                                  int64_t nsys, double atol, double rtol, int64_t* total_nsteps);
+
 static int legacy_n_const(int kind) {
     return kind == WIND_NET_KATZ96 ? 10 : (kind == WIND_NET_NR_TEST ? 4 : 2);
 }
@@ -74,17 +79,6 @@ int cudaIntegrateSystem(float tnow, float tend, int n_integration_steps, float* 
                         float* equations, int Nsystems, int Nequations_per_system,
                         float ABSOLUTE, float RELATIVE) {
     if (Nsystems <= 0) return 0;
-    const int N = Nequations_per_system;
-    const int nc = legacy_n_const(WIND_LEGACY_NET);
-    std::vector<double> c((size_t)Nsystems * nc), y((size_t)Nsystems * N);
-    for (size_t i = 0; i < c.size(); i++) c[i] = constants[i];
-    for (size_t i = 0; i < y.size(); i++) y[i] = equations[i];
-    wind_network net;
-    std::memset(&net, 0, sizeof(net));
-    net.kind = WIND_LEGACY_NET;
-    net.n_eq = N;
-    net.n_const = nc;
-    net.constants = c.data();
     wind_options o;
     wind_default_options(&o);
     o.method = WIND_LEGACY_METHOD;
@@ -96,11 +90,9 @@ int cudaIntegrateSystem(float tnow, float tend, int n_integration_steps, float* 
     if (const char* s = std::getenv("WIND_LEGACY_CONTROLLER"))
         if (!std::strcmp(s, "gold")) o.controller = WIND_CTRL_GOLD;
     int64_t total = 0;
-    const int st = wind_integrate(&o, &net, (double)tnow, (double)tend, n_integration_steps,
-                                  y.data(), Nsystems, (double)ABSOLUTE, (double)RELATIVE, nullptr,
-                                  nullptr, &total, WIND_MEM_HOST, nullptr);
-    if (st != WIND_OK) return -1;
-    for (size_t i = 0; i < y.size(); i++) equations[i] = (float)y[i];
-    return (int)total;
+    const int st = wind_integrate_f32(&o, WIND_LEGACY_NET, Nequations_per_system, legacy_n_const(WIND_LEGACY_NET),
+                                      (double)tnow, (double)tend, n_integration_steps, constants, equations,
+                                      Nsystems, (double)ABSOLUTE, (double)RELATIVE, &total);
+    return st == WIND_OK ? (int)total : -1;
 }
 #endif
