@@ -38,6 +38,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "reaction_words.cuh"
 #include "solvers_reg.cuh"
 #include "warp_kernel.cuh"
 
@@ -47,21 +48,6 @@ namespace wind {
 // +-1 or +-2; exact): a reaction takes its reactants by one s and makes its
 // products by another, so two entries per reaction hold them all, and two more
 // serve s = 0 and padding.
-// An incidence of a species, or a term of a Jacobian entry, in one word: the
-// signed rate's byte offset (19 bits), two species (6 bits each: reactants a and
-// b of an incidence, the other reactant and the column of a term), and whether
-// the term is its entry's last.
-constexpr uint32_t LU_LAST = 1u << 31;
-__device__ __forceinline__ uint32_t lu_pack(int slot, int first, int second) {
-    return (uint32_t)(slot * 8) | ((uint32_t)first << 19) | ((uint32_t)second << 25);
-}
-__device__ __forceinline__ double lu_at(const double* base, uint32_t bytes) {
-    return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(base) + bytes);
-}
-__device__ __forceinline__ double lu_rate(const double* rates, uint32_t q) { return lu_at(rates, q & 0x7ffffu); }
-__device__ __forceinline__ uint32_t lu_first(uint32_t q) { return (q >> 16) & 0x1f8u; }   // byte offsets
-__device__ __forceinline__ uint32_t lu_second(uint32_t q) { return (q >> 22) & 0x1f8u; }
-
 struct LuLayout {
     // byte offsets inside one team's slice
     int rates, inc_off, inc, term_off, term, lt, vb, rows, rows2, pb, bytes;
@@ -137,8 +123,8 @@ __device__ __forceinline__ double lu_rhs(const Ctx& c, int r) {
         double g[4], vb[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            g[u] = __dmul_rn(lu_rate(c.rates, q[u]), lu_at(c.vb, lu_first(q[u])));
-            vb[u] = lu_at(c.vb, lu_second(q[u]));
+            g[u] = __dmul_rn(rx_rate(c.rates, q[u]), rx_at(c.vb, rx_first(q[u])));
+            vb[u] = rx_at(c.vb, rx_second(q[u]));
         }
         acc = fma(g[0], vb[0], acc);
         acc2 = fma(g[1], vb[1], acc2);
@@ -164,15 +150,15 @@ __device__ __forceinline__ void lu_jac_row(const Ctx& c, int r) {
         double ks[4], v[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            ks[u] = lu_rate(c.rates, q[u]);
-            v[u] = lu_at(c.vb, lu_first(q[u]));
+            ks[u] = rx_rate(c.rates, q[u]);
+            v[u] = rx_at(c.vb, rx_first(q[u]));
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             // an entry's partial sums are stored over until its last term
             acc = fma(ks[u], v[u], acc);
-            *reinterpret_cast<double*>(reinterpret_cast<char*>(row) + lu_second(q[u])) = acc;
-            acc = (q[u] & LU_LAST) ? 0.0 : acc;
+            *reinterpret_cast<double*>(reinterpret_cast<char*>(row) + rx_second(q[u])) = acc;
+            acc = (q[u] & RX_MARK) ? 0.0 : acc;
         }
     }
 }
@@ -394,7 +380,7 @@ __device__ __forceinline__ bool lu_stage(const LuCtx<L, COLS>& c, const KParams&
             const int st = stoich(j, a, b, cc, d);
             int slot = st < 0 ? 2 * r : 2 * r + 1;
             if (st == 0) slot = finite64(rates[2 * r]) || finite64(rates[2 * r + 1]) ? 2 * R : 2 * R + 1;  // 0 * k
-            inc[o++] = lu_pack(slot, a, b);
+            inc[o++] = rx_pack(slot, a, b);
         }
         // d w / d y_a = k y_b, then d w / d y_b = k y_a, per column in list order
         const int e0 = inc_off[j];
@@ -403,16 +389,16 @@ __device__ __forceinline__ bool lu_stage(const LuCtx<L, COLS>& c, const KParams&
             const int t0 = t;
             for (int e = e0; e < o; e++) {
                 const uint32_t q = inc[e];
-                const int slot = (int)(q & 0x7ffffu) >> 3, a = (int)(lu_first(q) >> 3), b = (int)(lu_second(q) >> 3);
+                const int slot = (int)(q & 0x7ffffu) >> 3, a = (int)(rx_first(q) >> 3), b = (int)(rx_second(q) >> 3);
                 if (slot >= 2 * R) continue;
-                if (a == col) term[t++] = lu_pack(slot, b, col);
-                if (b == col) term[t++] = lu_pack(slot, a, col);
+                if (a == col) term[t++] = rx_pack(slot, b, col);
+                if (b == col) term[t++] = rx_pack(slot, a, col);
             }
-            if (t > t0) term[t - 1] |= LU_LAST;
+            if (t > t0) term[t - 1] |= RX_MARK;
         }
         // padding: rate zero, the zero beside the state, the column beside the row
-        while (o < inc_off[j + 1]) inc[o++] = lu_pack(2 * R, COLS, COLS);
-        while (t < term_off[j + 1]) term[t++] = lu_pack(2 * R, COLS, COLS);
+        while (o < inc_off[j + 1]) inc[o++] = rx_pack(2 * R, COLS, COLS);
+        while (t < term_off[j + 1]) term[t++] = rx_pack(2 * R, COLS, COLS);
         if (LT) {
             const float* Lg = p.linear + s * (int64_t)N * N;
             for (int k = 0; k < N; k++) LT[k * N + j] = Lg[j * N + k];

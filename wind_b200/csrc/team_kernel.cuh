@@ -23,12 +23,15 @@
 // s is not zero.  A pivot that is zero or not finite, or a result that is not
 // finite, sends the substep to the full-width elimination (team_gje_general).
 //
+// Both passes are loops of one step's code (two widths), the rows moving up one
+// register per step: unrolled they were 2,000 instructions at N = 16 and 6,000 at
+// N = 32, and waited for instruction fetch (68,800 cycles a solve with 1,500
+// systems of 32 species on the GPU, now 30,300; 14,000 and 11,800 with 1,000 of 16).
+//
 // What bounds it: the chain of N pivot steps (hand-over through shared memory,
-// one division, the first update) and the lane's incidence list.  The full-width
-// row form this replaced spent about 130 us per substep at N = 16, in 2N
-// divisions by one lane per step and in instruction fetch: 1,000 systems of 16
-// species (160 reactions, dt = 1e-3, atol = rtol = 5e-3) took 219.4 ms, now
-// 16.4 ms.
+// one division, the first update).  1,000 systems of 16 species (160 reactions,
+// dt = 1e-3, atol = rtol = 5e-3): 219.4 ms with the full-width row form (2N
+// divisions by one lane per step), 16.4 ms by columns, 12.8 ms now.
 //
 // One loop turn is one substep of every team of the warp, whatever part of its
 // attempt the team is in, so teams never wait for each other's attempts or
@@ -39,35 +42,31 @@
 
 #include "common.cuh"
 #include "networks.cuh"
+#include "reaction_words.cuh"
 
 namespace wind {
 
 constexpr int TEAM_MAXN = 32;
 
-// An incidence of species l: reaction id, reactants a and b, and how often l
-// is consumed (nn) and produced (np) by it.
-__device__ __forceinline__ uint32_t team_pack(int rr, int a, int b, int nn, int np) {
-    return (uint32_t)rr | ((uint32_t)a << 16) | ((uint32_t)b << 21) | ((uint32_t)nn << 26) |
-           ((uint32_t)np << 28);
-}
-
 struct TeamLayout {
     // byte offsets inside one team's shared slice: the Jacobian at the
     // accepted state, the Jacobian of the second half step / the columns handed
-    // over by the elimination (SIE only), vectors, the dense term, rates and
-    // incidence lists
-    int jy, w, vec, lt, rates, inc_off, inc, bytes;
+    // over by the elimination (SIE only), vectors (the state followed by a zero),
+    // the dense term, signed rates, unit lists and (SIE) Jacobian terms
+    int jy, w, vec, lt, rates, inc_off, inc, term_off, term, bytes;
     __host__ __device__ static int align16(int x) { return (x + 15) & ~15; }
     __host__ __device__ TeamLayout(int nmax, int R, bool lin, bool matrices) {
         const int mat = matrices ? nmax * nmax * 8 : 0;
         int off = 0;
         jy = off; off = align16(off + mat);
-        w = off; off = align16(off + mat);
-        vec = off; off = align16(off + 2 * nmax * 8);
+        w = off; off = align16(off + mat + (matrices ? 2 * nmax * 8 : 0));  // and two exchange rows
+        vec = off; off = align16(off + (2 * nmax + 2) * 8);
         lt = off; off = align16(off + (lin ? nmax * nmax * 4 : 0));
-        rates = off; off = align16(off + R * 8);
+        rates = off; off = align16(off + (2 * R + 1) * 8);
         inc_off = off; off = align16(off + (nmax + 1) * 4);
-        inc = off; off = align16(off + 4 * R * 4);
+        inc = off; off = align16(off + (4 * R + 3 * nmax + 4) * 4);     // and the word read ahead
+        term_off = off; off = align16(off + (matrices ? (nmax + 1) * 4 : 0));
+        term = off; off = align16(off + (matrices ? (8 * R + 3 * nmax + 4) * 4 : 0));
         bytes = off;
     }
 };
@@ -86,65 +85,72 @@ struct TeamCtx {
     double* v;      // [NMAX] state being stepped
     double* f;      // [NMAX] RHS at v
     const float* LT;   // [NMAX*NMAX] LT[i*NMAX+j] = L[j][i], or null
-    const double* rates;      // [R]
+    const double* rates;      // [2R + 1]: -k, k of each reaction, 0
     const int* inc_off;       // [NMAX+1] CSR offsets
-    const uint32_t* inc;      // packed incidences (team_pack)
+    const uint32_t* inc;      // unit list: one word per -w or +w of f_l
+    const int* term_off;
+    const uint32_t* term;     // one word per unit of a Jacobian entry, by column
 };
 
-// x - d (nn times), then x + d (np times), nn + np >= 1, each rounded.
-__device__ __forceinline__ xd team_apply(xd x, xd d, int nn, int np) {
-    x = x + (nn ? -d : d);
-    if (nn + np > 1) {
-        x = x + (nn == 2 ? -d : d);
-        if (nn + np > 2) {
-            x = x + d;
-            if (nn + np > 3) x = x + d;
-        }
-    }
-    return x;
-}
-
-// f_l and, with JAC, column l of Jt into J, for the current v.  The loads of
-// four incidences are in flight before the first is used.
+// f_l and, with JAC, column l of Jt into J, for the current v.  The contract's
+// updates are the units x - d and x + d, that is x + (-d) and x + d: the lists
+// hold one word per unit with the signed rate, f's in reaction order, the
+// Jacobian's by entry (each entry's units in the order of the contract, from the
+// dense term on), so an entry is summed in a register and stored without being
+// read back.  Padded to four words that add zero; the next four are in flight.
+// (Scanning a list of reactions and updating entries in place took 400 cycles a
+// reaction.)
 template <int NMAX, bool JAC>
 __device__ __forceinline__ void team_rhs_jac(const TeamCtx<NMAX>& c, double* J) {
     const int l = c.l;
     if (l < c.N) {
         xd acc = 0.0;
-        if (c.LT) {
+        if (c.LT)
             for (int k = 0; k < c.N; k++) acc += xd((double)c.LT[k * NMAX + l]) * xd(c.v[k]);
-            if (JAC)
-                for (int i = 0; i < c.N; i++) J[i * NMAX + l] = (double)c.LT[i * NMAX + l];
-        } else if (JAC) {
-            for (int i = 0; i < c.N; i++) J[i * NMAX + l] = 0.0;
-        }
-        const int e1 = c.inc_off[l + 1];
-        for (int e = c.inc_off[l]; e < e1; e += 4) {
-            uint32_t q[4];
-            double k[4], ya[4], yb[4];
+        {
+            const int e1 = c.inc_off[l + 1];
+            int e = c.inc_off[l];
+            uint4 next = *reinterpret_cast<const uint4*>(c.inc + e);
+            for (; e < e1; e += 4) {
+                const uint32_t q[4] = {next.x, next.y, next.z, next.w};
+                next = *reinterpret_cast<const uint4*>(c.inc + e + 4);
+                xd w[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                q[u] = c.inc[e + u < e1 ? e + u : e];
-                k[u] = c.rates[q[u] & 0xffffu];
-                ya[u] = c.v[(q[u] >> 16) & 31u];
-                yb[u] = c.v[(q[u] >> 21) & 31u];
-            }
+                for (int u = 0; u < 4; u++)
+                    w[u] = xd(rx_rate(c.rates, q[u])) * xd(rx_at(c.v, rx_first(q[u]))) *
+                           xd(rx_at(c.v, rx_second(q[u])));
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (e + u < e1) {
-                    const int nn = (q[u] >> 26) & 3, np = q[u] >> 28;
-                    const xd db = xd(k[u]) * xd(ya[u]);
-                    acc = team_apply(acc, db * xd(yb[u]), nn, np);
-                    if (JAC) {
-                        double* ra = J + ((q[u] >> 16) & 31u) * NMAX + l;
-                        double* rb = J + ((q[u] >> 21) & 31u) * NMAX + l;
-                        *ra = team_apply(*ra, xd(k[u]) * xd(yb[u]), nn, np).v;
-                        *rb = team_apply(*rb, db, nn, np).v;
-                    }
-                }
+                for (int u = 0; u < 4; u++) acc += w[u];
             }
         }
         c.f[l] = acc.v;
+        if (JAC) {
+            for (int i = 0; i < c.N; i++) J[i * NMAX + l] = c.LT ? (double)c.LT[i * NMAX + l] : 0.0;
+            const int e1 = c.term_off[l + 1];
+            int e = c.term_off[l];
+            uint4 next = *reinterpret_cast<const uint4*>(c.term + e);
+            xd sum = 0.0;
+            for (; e < e1; e += 4) {
+                const uint32_t q[4] = {next.x, next.y, next.z, next.w};
+                next = *reinterpret_cast<const uint4*>(c.term + e + 4);
+                xd d[4];
+                double start[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    d[u] = xd(rx_rate(c.rates, q[u])) * xd(rx_at(c.v, rx_first(q[u])));
+                    // (padding's column is NMAX: no dense entry)
+                    start[u] = 0.0;
+                    if (c.LT && rx_second(q[u]) < 8u * NMAX)
+                        start[u] = (double)c.LT[(rx_second(q[u]) >> 3) * NMAX + l];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    // an entry's partial sums are stored over until its last unit
+                    sum = ((q[u] & RX_MARK) ? xd(start[u]) : sum) + d[u];
+                    J[(rx_second(q[u]) >> 3) * NMAX + l] = sum.v;
+                }
+            }
+        }
     }
     team_sync(c.mask);
 }
@@ -184,11 +190,13 @@ struct TeamProduct {
 template <int NMAX, int CTRL>
 __device__ __noinline__ double team_gje_general(unsigned mask, int l, int leader, int N, double* jy, double* w,
                                                 double* v, double* f, const float* LT, const double* rates,
-                                                const int* inc_off, const uint32_t* inc, double h) {
+                                                const int* inc_off, const uint32_t* inc, const int* term_off,
+                                                const uint32_t* term, double h) {
     TeamCtx<NMAX> c;
     c.mask = mask; c.l = l; c.leader = leader; c.N = N;
     c.jy = jy; c.w = w; c.v = v; c.f = f;
     c.LT = LT; c.rates = rates; c.inc_off = inc_off; c.inc = inc;
+    c.term_off = term_off; c.term = term;
     team_rhs_jac<NMAX, true>(c, w);
     xd Mr[NMAX], Ir[NMAX];
 #pragma unroll
@@ -257,93 +265,143 @@ __device__ __noinline__ double team_gje_general(unsigned mask, int l, int leader
     return out;
 }
 
+// Steps [i0, i1) of the downward pass: x[k] holds row i + k of the lane's column,
+// W rows from the pivot row on.  The pivot lane hands over its column (row i in
+// F[0]), every lane divides its row-i entry, keeps it in X[i] and updates the rows
+// below, which move up one register: the loop is one step's code, however many
+// steps there are.
+template <int W, int NMAX>
+__device__ __forceinline__ bool team_gje_down(const TeamCtx<NMAX>& c, xd (&x)[NMAX], int i0, int i1) {
+    const int l = c.l;
+    double* X = c.w;
+    bool ok = true;
+#pragma unroll 1
+    for (int i = i0; i < i1; i++) {
+        double* F = c.w + NMAX * NMAX + (i & 1) * NMAX;
+        if (l == i) {
+#pragma unroll
+            for (int t = 0; t < W; t += 2) *reinterpret_cast<double2*>(F + t) = make_double2(x[t].v, x[t + 1].v);
+#pragma unroll
+            for (int t = 0; t < W; t++) x[t] = (t == 0) ? 1.0 : 0.0;  // column i of Inv starts
+        }
+        team_sync(c.mask);
+        const double2 f01 = *reinterpret_cast<const double2*>(F);
+        const xd s = f01.x;
+        ok = ok && s.v != 0.0 && finite64(s.v);
+        const xd xi = x[0] / s;
+        X[i * NMAX + l] = xi.v;
+        x[0] = x[1] - xd(f01.y) * xi;
+#pragma unroll
+        for (int k = 2; k < W; k += 2) {
+            const double2 f = *reinterpret_cast<const double2*>(F + k);
+            x[k - 1] = x[k] - xd(f.x) * xi;
+            x[k] = x[k + 1] - xd(f.y) * xi;
+        }
+        x[W - 1] = 0.0;
+    }
+    return ok;
+}
+
+// Steps b1 >= b > b0 of the upward pass: x[k] holds row b - k of the lane's
+// column of Inv.  Row b is final and goes to X[b]; M's entries above the pivot
+// stand in column b of X.  (Rows below zero read what precedes X and are not used.)
+template <int W, int NMAX>
+__device__ __forceinline__ void team_gje_up(const TeamCtx<NMAX>& c, xd (&x)[NMAX], int b1, int b0) {
+    const int l = c.l;
+    double* X = c.w;
+#pragma unroll 1
+    for (int b = b1; b > b0; b--) {
+        const double* col = X + b * NMAX + b;
+        const xd xb = x[0];
+#pragma unroll
+        for (int k = 1; k < W; k++) x[k - 1] = x[k] - xd(col[-k * NMAX]) * xb;
+        x[W - 1] = 0.0;
+        team_sync(c.mask);  // column entries of row b are read before the row is replaced
+        X[b * NMAX + l] = xb.v;
+    }
+}
+
 // One SIE substep of size h from the state in v with f in f and Jt in J (jy
 // or w); returns the stepped component l.  Column form of the file comment.
 // `clean` is cleared when the full-width elimination had to be used, which
 // overwrites jy.
 template <int NMAX, int CTRL>
 __device__ __forceinline__ double team_gje_step(const TeamCtx<NMAX>& c, const double* J, double h, bool& clean) {
+    constexpr int H = NMAX > 8 ? NMAX / 2 : NMAX;  // rows of the second half's steps
     const int l = c.l, N = c.N;
-    double* F = c.w;  // columns handed over, [step][row]
+    double* X = c.w;  // rows as they leave the downward pass, then Inv
     xd x[NMAX];
 #pragma unroll
     for (int t = 0; t < NMAX; t++)
         x[t] = team_matrix_elem<CTRL>((l < N && t < N) ? J[t * NMAX + l] : 0.0, h, t == l);
-    bool ok = true;
     team_sync(c.mask);  // J may be w: every column is in registers before the first is handed over
+    const int mid = min(N, NMAX - H);
+    bool ok = team_gje_down<NMAX>(c, x, 0, mid);
+    if (N > NMAX - H) ok = team_gje_down<H>(c, x, mid, N) && ok;
+    team_sync(c.mask);
 #pragma unroll
-    for (int i = 0; i < NMAX; i++) {
-        if (i < N) {
-            double* Fi = F + i * NMAX;
-            if (l == i) {
-#pragma unroll
-                for (int t = 0; t < NMAX; t += 2)
-                    *reinterpret_cast<double2*>(Fi + t) = make_double2(x[t].v, x[t + 1].v);
-#pragma unroll
-                for (int t = 0; t < NMAX; t++) x[t] = (t == i) ? 1.0 : 0.0;  // column i of Inv starts
-            }
-            team_sync(c.mask);
-            const xd s = Fi[i];
-            ok = ok && s.v != 0.0 && finite64(s.v);
-            x[i] = x[i] / s;
-#pragma unroll
-            for (int k = i + 1; k < NMAX; k++) x[k] -= xd(Fi[k]) * x[i];
-        }
+    for (int t = 0; t < NMAX; t++) {
+        const int row = N - 1 - t;
+        x[t] = (row >= 0 && l <= row) ? X[row * NMAX + l] : 0.0;
     }
-#pragma unroll
-    for (int b = NMAX - 1; b > 0; b--) {
-        if (b < N) {
-            const double* Fb = F + b * NMAX;
-#pragma unroll
-            for (int k = 0; k < b; k++) x[k] -= xd(Fb[k]) * x[b];
-        }
-    }
+    team_sync(c.mask);
+    if (N > H) team_gje_up<NMAX>(c, x, N - 1, H - 1);
+    team_gje_up<H>(c, x, min(N, H) - 1, 0);
+    X[l] = x[0].v;
     double out = 0.0;
     if (l < N) {
         TeamProduct<CTRL> prod(c.v[l], h);
-#pragma unroll
-        for (int k = 0; k < NMAX; k++)
-            if (k < N) prod.add(x[k], c.f[k]);
+        for (int k = 0; k < N; k++) prod.add(X[k * NMAX + l], c.f[k]);
         out = prod.result(c.v[l]);
         ok = ok && finite64(out);
     }
     if (!__all_sync(c.mask, ok)) {
         out = team_gje_general<NMAX, CTRL>(c.mask, l, c.leader, N, c.jy, c.w, c.v, c.f, c.LT, c.rates,
-                                           c.inc_off, c.inc, h);
+                                           c.inc_off, c.inc, c.term_off, c.term, h);
         clean = false;
     }
     return out;
 }
 
-// Stage system s: rates, the dense term transposed, and the per-species
-// incidence lists (reaction ids ascending).  A species index >= N marks the
-// system BAD_INPUT (returned) and nothing of it is read again.
-template <int NMAX>
+// Stage system s: signed rates, the dense term transposed, the unit lists and,
+// with JAC, the Jacobian terms.  A species index >= N marks the system BAD_INPUT
+// (returned) and nothing of it is read again.
+template <int NMAX, bool JAC>
 __device__ __forceinline__ bool team_stage(const TeamCtx<NMAX>& c, const KParams& p, int64_t s, double* rates,
-                                           int* inc_off, uint32_t* inc, float* LT) {
+                                           int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, float* LT) {
     const int N = c.N, R = p.n_react, l = c.l;
     const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * R;
     bool bad = false;
     for (int r = l; r < R; r += NMAX) {
-        rates[r] = p.rates[s * R + r];
+        const double k = p.rates[s * R + r];
+        rates[2 * r] = -k;
+        rates[2 * r + 1] = k;
         const uint2 q = __ldg(sp + r);
         const unsigned nn = (unsigned)N;
         bad = bad || (q.x & 0xffffu) >= nn || (q.x >> 16) >= nn || (q.y & 0xffffu) >= nn || (q.y >> 16) >= nn;
     }
     if (__any_sync(c.mask, bad)) return true;
-    const unsigned ul = (unsigned)l;
+    // units of species l in reaction (a, b -> cc, d): nn times -, then np times +
     if (l < N) {
         int cnt = 0;
         for (int r = 0; r < R; r++) {
             const uint2 q = __ldg(sp + r);
-            cnt += ((q.x & 0xffffu) == ul) | ((q.x >> 16) == ul) | ((q.y & 0xffffu) == ul) | ((q.y >> 16) == ul);
+            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+            cnt += (a == l) + (b == l) + (cc == l) + (d == l);
         }
-        inc_off[l + 1] = cnt;
+        inc_off[l + 1] = (cnt + 3) & ~3;
+        if (JAC) term_off[l + 1] = (2 * cnt + 3) & ~3;
     }
     team_sync(c.mask);
     if (l == 0) {
         inc_off[0] = 0;
         for (int j = 0; j < N; j++) inc_off[j + 1] += inc_off[j];
+        if (JAC) {
+            term_off[0] = 0;
+            for (int j = 0; j < N; j++) term_off[j + 1] += term_off[j];
+        }
+        rates[2 * R] = 0.0;
+        c.v[NMAX] = 0.0;
     }
     team_sync(c.mask);
     if (l < N) {
@@ -352,8 +410,30 @@ __device__ __forceinline__ bool team_stage(const TeamCtx<NMAX>& c, const KParams
             const uint2 q = __ldg(sp + r);
             const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
             const int nn = (a == l) + (b == l), np = (cc == l) + (d == l);
-            if (nn + np) inc[o++] = team_pack(r, a, b, nn, np);
+            for (int u = 0; u < nn + np; u++) inc[o++] = rx_pack(2 * r + (u >= nn), a, b);
         }
+        if (JAC) {
+            // d w / d y_a = k y_b, then d w / d y_b = k y_a: per reaction all
+            // units of the first before the second
+            int t = term_off[l];
+            for (int col = 0; col < N; col++) {
+                const int t0 = t;
+                for (int e = inc_off[l]; e < o;) {
+                    const uint32_t q = inc[e];
+                    const int r = (int)(q & 0x7ffffu) >> 4, a = (int)(rx_first(q) >> 3), b = (int)(rx_second(q) >> 3);
+                    int n = e + 1;  // the reaction's units are neighbours
+                    while (n < o && ((int)(inc[n] & 0x7ffffu) >> 4) == r) n++;
+                    if (a == col)
+                        for (int u = e; u < n; u++) term[t++] = rx_pack((int)(inc[u] & 0x7ffffu) >> 3, b, col);
+                    if (b == col)
+                        for (int u = e; u < n; u++) term[t++] = rx_pack((int)(inc[u] & 0x7ffffu) >> 3, a, col);
+                    e = n;
+                }
+                if (t > t0) term[t0] |= RX_MARK;
+            }
+            while (t < term_off[l + 1]) term[t++] = rx_pack(2 * R, NMAX, NMAX) | RX_MARK;
+        }
+        while (o < inc_off[l + 1]) inc[o++] = rx_pack(2 * R, NMAX, NMAX);
         if (LT) {
             const float* Lg = p.linear + s * (int64_t)N * N;
             for (int k = 0; k < N; k++) LT[k * NMAX + l] = Lg[l * N + k];
@@ -384,7 +464,7 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
     c.jy = reinterpret_cast<double*>(base + lay.jy);
     c.w = reinterpret_cast<double*>(base + lay.w);
     c.v = reinterpret_cast<double*>(base + lay.vec);
-    c.f = c.v + NMAX;
+    c.f = c.v + NMAX + 2;
     float* LT = lin ? reinterpret_cast<float*>(base + lay.lt) : nullptr;
     double* rates = reinterpret_cast<double*>(base + lay.rates);
     int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
@@ -393,6 +473,10 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
     c.rates = rates;
     c.inc_off = inc_off;
     c.inc = inc;
+    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
+    uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
+    c.term_off = term_off;
+    c.term = term;
     const int N = c.N, l = c.l;
     const uint64_t t_start = p.timeout_ns ? global_ns() : 0;
     const double tend = p.tend;
@@ -415,7 +499,7 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
                 if (l == 0) ticket = atomicAdd(&p.counters[CNT_QUEUE], 1ull);
                 s = (int64_t)__shfl_sync(c.mask, ticket, c.leader);
                 if (s >= p.nsys) return;
-                stop = team_stage<NMAX>(c, p, s, rates, inc_off, inc, LT);
+                stop = team_stage<NMAX, SIE>(c, p, s, rates, inc_off, inc, term_off, term, LT);
                 st = stop ? WIND_SYS_BAD_INPUT : WIND_SYS_OK;
                 y = (l < N) ? p.y[s * N + l] : 0.0;
                 tnow = p.tnow;
