@@ -33,6 +33,14 @@
 // stored without being read back.  Lists are padded to whole 16-byte words of
 // four with entries that add zero.
 //
+// The dense term is widened to FP64 when a system is staged: a substep reads
+// each entry twice, and a conversion takes 12 to 24 cycles of a unit that the
+// pivot keys and reciprocals need too.  3,000 dense systems of 32 species and
+// 64 reactions: 704 to 637 ms (893 before this kernel).  The 4 KB a team that this costs take teams
+// away where there are many reactions, and the gain is smaller there: at looser
+// tolerances 68.3 to 62.0 ms with 64 reactions, 79.6 to 76.0 ms with 160, 92.7
+// to 91.3 ms with 240.
+//
 // The values are those of the one-row-per-lane kernel this replaced, bit for
 // bit: the same pivots, multipliers and order of every sum.
 #pragma once
@@ -59,7 +67,7 @@ struct LuLayout {
         inc = off; off = align16(off + (4 * R + 3 * n + 4) * 4);  // and the word read ahead
         term_off = off; off = align16(off + (n + 1) * 4);
         term = off; off = align16(off + (8 * R + 3 * n + 4) * 4);
-        lt = off; off = align16(off + (lin ? n * n * 4 : 0));
+        lt = off; off = align16(off + (lin ? n * n * 8 : 0));     // dense term, widened once
         vb = off; off = align16(off + (cols + 1) * 8);           // state, and a zero
         // Jacobian rows: at the accepted state, and at the half step -- of up
         // to 16 species a second set is small beside the lists, and keeps the
@@ -84,7 +92,7 @@ struct LuCtx {
     const uint32_t* inc;
     const int* term_off;
     const uint32_t* term;
-    const float* LT;   // LT[k*N + r] = L[r][k], or null
+    const double* LT;  // LT[k*N + r] = L[r][k], or null
     double* vb;
     double* rows;      // Jacobian rows in use
     double* pb;
@@ -93,16 +101,16 @@ struct LuCtx {
 // sum_k L[r][k] w[k] for the dense term (w in shared memory, FP64), four
 // independent accumulators over a compile-time column loop.
 template <int COLS>
-__device__ __forceinline__ double lu_dense_dot(const float* LT, const double* w, int r, int N) {
+__device__ __forceinline__ double lu_dense_dot(const double* LT, const double* w, int r, int N) {
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
     for (int k = 0; k < COLS; k += 4) {
         if (k < N) {
             const double2 w01 = *reinterpret_cast<const double2*>(w + k);
-            s0 = fma((double)LT[k * N + r], w01.x, s0);
-            if (k + 1 < N) s1 = fma((double)LT[(k + 1) * N + r], w01.y, s1);
-            if (k + 2 < N) s2 = fma((double)LT[(k + 2) * N + r], w[k + 2], s2);
-            if (k + 3 < N) s3 = fma((double)LT[(k + 3) * N + r], w[k + 3], s3);
+            s0 = fma(LT[k * N + r], w01.x, s0);
+            if (k + 1 < N) s1 = fma(LT[(k + 1) * N + r], w01.y, s1);
+            if (k + 2 < N) s2 = fma(LT[(k + 2) * N + r], w[k + 2], s2);
+            if (k + 3 < N) s3 = fma(LT[(k + 3) * N + r], w[k + 3], s3);
         }
     }
     return (s0 + s1) + (s2 + s3);
@@ -179,7 +187,7 @@ __device__ __forceinline__ void lu_load_row(const Ctx& c, int r, double h, doubl
         for (int q = 0; q < 2; q++) {
             const int t = t0 + q;
             double j = q ? w.y : w.x;
-            if (c.LT && t < c.N) j += (double)c.LT[t * c.N + r];
+            if (c.LT && t < c.N) j += c.LT[t * c.N + r];
             a[t] = (t == r) ? fma(-h, j, 1.0) : -h * j;
         }
     }
@@ -301,23 +309,27 @@ __device__ __forceinline__ double lu_solve(const LuCtx<L, COLS>& c, double (&a)[
     if constexpr (COLS > 24) lu_steps<24, COLS, GUARD, EXACT>(c, a, b, pv);
     __syncwarp();  // the last pivot row is read before the next solve publishes
     // back substitution by columns: x_i from the lane that pivoted at step i
-    double x = 0.0;
 #pragma unroll
-    for (int i = COLS - 1; i >= 0; i--) {
+    for (int i = COLS - 1; i > 0; i--) {
         if ((!GUARD && i <= COLS - 4) || i < N) {
             const int p = (pv.rows[i / 6] >> (5 * (i % 6))) & 31;
             const double xi = __shfl_sync(0xffffffffu, b * pv.rcp, c.leader + (p & (L - 1)));
             const double u = fma(-a[i], xi, b);
             b = (pv.step >= 0 && pv.step < i) ? u : b;
-            if (l == i) x = xi;
         }
     }
-    return x;
+    // component l is the pivot row's of step l
+    uint32_t w = pv.rows[0];
+#pragma unroll
+    for (int q = 1; q < (COLS + 5) / 6; q++) w = (l >= 6 * q) ? pv.rows[q] : w;
+    const int p = (int)(w >> (5 * (l % 6)));
+    const double x = __shfl_sync(0xffffffffu, b * pv.rcp, c.leader + (p & (L - 1)));
+    return l < N ? x : 0.0;
 }
 
 // The solve with selected updates, for solutions that are not finite.
 template <bool GUARD, int L, int COLS>
-__device__ __noinline__ double lu_solve_exact(int l, int leader, int N, int tm, bool live, const float* LT,
+__device__ __noinline__ double lu_solve_exact(int l, int leader, int N, int tm, bool live, const double* LT,
                                               double* rows, double* pb, double h, double f) {
     LuCtx<L, COLS> c;
     c.l = l; c.leader = leader; c.N = N; c.tm = tm; c.live = live;
@@ -332,7 +344,7 @@ __device__ __noinline__ double lu_solve_exact(int l, int leader, int N, int tm, 
 // (returned) and nothing of it is read again.
 template <int L, int COLS>
 __device__ __forceinline__ bool lu_stage(const LuCtx<L, COLS>& c, const KParams& p, int64_t s, double* rates,
-                                         int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, float* LT) {
+                                         int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, double* LT) {
     const int N = c.N, R = p.n_react, l = c.l;
     const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * R;
     bool bad = false;
@@ -445,7 +457,7 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
     uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
     int* term_off = reinterpret_cast<int*>(base + lay.term_off);
     uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
-    float* LT = lin ? reinterpret_cast<float*>(base + lay.lt) : nullptr;
+    double* LT = lin ? reinterpret_cast<double*>(base + lay.lt) : nullptr;
     c.rates = rates;
     c.inc_off = inc_off;
     c.inc = inc;
