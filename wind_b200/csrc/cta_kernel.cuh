@@ -173,7 +173,11 @@ struct CtaCtx {
     int* piv;    // logical row -> physical row
     int* act;    // active rows of the trailing update
     int* misc;   // warp counts [CTA_WARPS]
-    unsigned long long* best;  // pivot vote, three rotating slots
+    unsigned long long* best;  // pivot vote, three rotating slots (in misc, behind the counts)
+    // CTA-wide maxima (float bits), three rotating slots.  A vote leaves its last
+    // pivot in `best`, and a refinement right behind it may start in any slot: the
+    // two share no word.
+    unsigned maxima[3];
     void* cand;  // CtaCand<T>[2][CTA_WARPS]
     // tensor-core rank updates (MIXED_TC): accumulator base in tensor
     // memory, completion mbarrier, operand staging, columns rounded to 16
@@ -731,15 +735,11 @@ __device__ void cta_solve(const T* A) {
 }
 
 // ---- MIXED: FP32 Gauss-Jordan inverse reused across an attempt ----------
-// misc[] slots 8..10: rotating CTA-wide maxima (unsigned float bits).
-constexpr int CTA_MAXSLOT = 8;
-
 // CTA-wide max of |v| (one barrier).  `phase` rotates over three slots; the
 // slot of the next call is cleared here -- its last readers read it two
 // calls ago, before the barrier of the previous call.
 __device__ __forceinline__ double cta_max_abs(double v, int& phase) {
-    const CtaCtx& c = cta_ctx;
-    unsigned* slot = reinterpret_cast<unsigned*>(c.misc + CTA_MAXSLOT);
+    unsigned* slot = cta_ctx.maxima;
     const unsigned w = __reduce_max_sync(0xffffffffu, fmax_bits(v));
     if (((int)threadIdx.x & 31) == 0) atomicMax(slot + phase, w);
     if ((int)threadIdx.x == 0) slot[(phase + 1) % 3] = 0u;
@@ -1654,7 +1654,7 @@ __device__ __forceinline__ void cta_run(const KParams& p, unsigned char* smem_ra
             }
         }
         double yl = own ? p.y[s * N + tid] : 0.0, y1l = 0.0, y2l = 0.0;
-        if (tid < 3) reinterpret_cast<unsigned*>(c.misc + CTA_MAXSLOT)[tid] = 0u;
+        if (tid < 3) c.maxima[tid] = 0u;
         __syncthreads();
 
         double tnow = p.tnow;
