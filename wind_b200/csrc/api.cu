@@ -106,6 +106,28 @@ static int builtin_nc(int kind) {
     }
 }
 
+cudaError_t allow_block_smem(const void* fn) {
+    static std::mutex mu;
+    static std::vector<std::pair<const void*, int>> fixed;  // static shared memory of each kernel
+    int dev = 0, most = 0, used = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> g(mu);
+        for (const auto& f : fixed)
+            if (f.first == fn) used = f.second;
+        if (used < 0) {
+            cudaFuncAttributes fa{};
+            e = cudaFuncGetAttributes(&fa, fn);
+            if (e != cudaSuccess) return e;
+            used = (int)fa.sharedSizeBytes;
+            fixed.push_back({fn, used});
+        }
+    }
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - used);
+}
+
 int device_sm_count() {
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 148;

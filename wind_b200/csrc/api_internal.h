@@ -79,6 +79,12 @@ inline wind_status cuda_status(cudaError_t e, const char* where) {
 // Status of the launch just issued.
 inline wind_status launch_status(const char* where) { return cuda_status(cudaGetLastError(), where); }
 
+// Lets `fn` be launched on the current device with any dynamic shared memory a
+// block can have there.  The limit belongs to the kernel, not to a launch: every
+// caller sets the same largest value, so no thread's launch or occupancy query
+// finds the smaller one of another thread's size.
+cudaError_t allow_block_smem(const void* fn);
+
 // True for null or for memory a kernel may dereference (device or managed).
 inline bool device_ptr(const void* ptr) {
     if (!ptr) return true;

@@ -57,7 +57,7 @@ static int cta_blocks_per_sm(CtaFn fn, int threads, size_t smem) {
     for (auto& e : cache)
         if (e.first.first == (const void*)fn && e.first.second == smem && e.second.first == threads)
             return e.second.second;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    (void)allow_block_smem((const void*)fn);
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess) nb = 0;
     cache.push_back({{(const void*)fn, smem}, {threads, nb}});
@@ -127,9 +127,7 @@ size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int solver) 
 wind_status launch_cta(const CtaPlan& pl, const KParams& p, cudaStream_t stream, double* scratch) {
     if (pl.need && !scratch) return WIND_ERR_ARGUMENT;
     CtaFn fn = reinterpret_cast<CtaFn>(const_cast<void*>(pl.fn));
-    // set for this launch every time (the occupancy cache may come from a
-    // launch of the same kernel with another size)
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes) != cudaSuccess)
+    if (allow_block_smem(pl.fn) != cudaSuccess)
         return launch_status("k_cta shared-memory attribute");
     fn<<<pl.grid, pl.threads, pl.smem_bytes, stream>>>(p, pl.gstride ? scratch : nullptr, scratch ? pl.gstride : 0,
                                                         pl.smem_cap);

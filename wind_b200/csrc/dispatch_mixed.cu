@@ -79,7 +79,7 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
     }
     if (smem > (size_t)cap) return WIND_ERR_UNSUPPORTED;
     MixedFn fn = mixed_fn(o.method, o.controller, o.solver);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_block_smem((const void*)fn) != cudaSuccess)
         return launch_status("k_mixed shared-memory attribute");
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, MIXED_THREADS, smem) != cudaSuccess || nb < 1)

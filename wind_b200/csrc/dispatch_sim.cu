@@ -46,7 +46,7 @@ wind_status launch_sim(const wind_options& o, const KParams& p, cudaStream_t str
     const size_t smem = warp_smem_bytes(p.n_eq, p.n_react, p.linear != nullptr, WIND_SOLVER_LU_F64,
                                         WARP_THREADS);
     if (smem > 227 * 1024) return WIND_ERR_UNSUPPORTED;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_block_smem((const void*)fn) != cudaSuccess)
         return launch_status("k_sim_warp shared-memory attribute");
     const int nb = sim_blocks_per_sm(fn, WARP_THREADS, smem);
     if (nb < 1) return WIND_ERR_UNSUPPORTED;

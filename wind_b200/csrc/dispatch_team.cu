@@ -35,7 +35,7 @@ static int team_blocks_per_sm(TeamFn fn, size_t smem) {
     std::lock_guard<std::mutex> g(mu);
     for (auto& e : cache)
         if (e.first.first == (const void*)fn && e.first.second == smem) return e.second;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    (void)allow_block_smem((const void*)fn);
     int nb = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32, smem) != cudaSuccess || nb < 1) {
         (void)cudaGetLastError();
@@ -77,9 +77,7 @@ wind_status launch_team(const wind_options& o, const KParams& p, cudaStream_t st
     if (tpw == 0) return WIND_ERR_UNSUPPORTED;
     const size_t smem = (size_t)tpw * lay.bytes;
     const int grid = (int)std::min<int64_t>((p.nsys + tpw - 1) / tpw, resident);
-    // the attribute is per function, and the cached occupancy above may come
-    // from a launch with another size: set it for this launch every time
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_block_smem((const void*)fn) != cudaSuccess)
         return launch_status("k_team shared-memory attribute");
     fn<<<grid, 32, smem, stream>>>(p, tpw);
     g_launches++;

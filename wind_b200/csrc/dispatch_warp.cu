@@ -31,7 +31,7 @@ static int warp_blocks_per_sm(WarpFn fn, int threads, size_t smem) {
     for (auto& e : cache)
         if (e.first.first == (const void*)fn && e.first.second == smem && e.second.first == threads)
             return e.second.second;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    (void)allow_block_smem((const void*)fn);
     int nb = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem) != cudaSuccess || nb < 1) {
         (void)cudaGetLastError();
@@ -64,7 +64,7 @@ wind_status launch_warp(const wind_options& o, const KParams& p, cudaStream_t st
     const int64_t need = (p.nsys + teams - 1) / teams;
     const int64_t cap = (int64_t)nb * device_sm_count();
     const int grid = (int)(need < cap ? need : cap);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_block_smem((const void*)fn) != cudaSuccess)
         return launch_status("k_warp shared-memory attribute");
     fn<<<grid, threads, smem, stream>>>(p);
     g_launches++;
