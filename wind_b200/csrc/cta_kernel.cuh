@@ -81,9 +81,10 @@ struct CtaLayout {
     int vec, piv, act, misc, cand, tcs, lt, mat, inc_off, inc, rt, spc, bytes;
     bool mat_in_smem, inc_in_smem, data_in_smem;
     size_t g_mat, g_inc, g_doubles;  // global slot: offsets and size in doubles
-    // Reaction records (LU_F64 and MIXED): rec_cap records of 12 bytes, in shared
-    // memory at `rec` (rec_in_smem) or behind the global slot's other parts
-    // (g_rec, rec_doubles); a launch without that room goes without them.
+    // Reaction records (SIE with LU_F64 or MIXED; RK2 reads none): rec_cap records
+    // of 12 bytes, in shared memory at `rec` (rec_in_smem) or behind the global
+    // slot's other parts (g_rec, rec_doubles); a launch without that room goes
+    // without them.
     int rec_cap, rec;
     bool rec_in_smem;
     size_t g_rec, rec_doubles;
@@ -106,7 +107,8 @@ struct CtaLayout {
     __host__ __device__ static int tc_stage_bytes(int N) {
         return 64 + 4 * 4096 + 4 * ((N + 15) & ~15) * 32;
     }
-    __host__ __device__ CtaLayout(int N, int R, bool lin, int solver, int smem_cap, bool tc = false) {
+    __host__ __device__ CtaLayout(int N, int R, bool lin, int solver, int smem_cap, bool tc = false,
+                                  bool records = true) {
         esz = (solver == WIND_SOLVER_MIXED) ? 4 : 8;
         ld = row_stride(N, esz);
         cols = data_cols(N);
@@ -138,7 +140,7 @@ struct CtaLayout {
         data_in_smem = (spc + a16(R * 8)) <= smem_cap;
         if (data_in_smem) off = spc + a16(R * 8);
         // room for twice the average incidence count in every species' list
-        rec_cap = solver == WIND_SOLVER_GJE_F64 || R > CTA_REC_MAXR ? 0 : 8 * R + 8 * ((N + 31) & ~31);
+        rec_cap = !records || solver == WIND_SOLVER_GJE_F64 || R > CTA_REC_MAXR ? 0 : 8 * R + 8 * ((N + 31) & ~31);
         rec = off;
         rec_in_smem = rec_cap > 0 && off + 12 * rec_cap <= smem_cap;
         if (rec_in_smem) off = a16(off + 12 * rec_cap);
@@ -1480,7 +1482,7 @@ __device__ __forceinline__ void cta_run(const KParams& p, unsigned char* smem_ra
     const int N = p.n_eq, R = p.n_react, tid = threadIdx.x;
     const bool own = tid < N;
     const bool lin = p.linear != nullptr;
-    const CtaLayout lay(N, R, lin, SOLVER, smem_cap, TC);
+    const CtaLayout lay(N, R, lin, SOLVER, smem_cap, TC, METHOD == WIND_METHOD_SIE);
     CtaCtx& c = cta_ctx;
     double* gslot = gscratch ? gscratch + (size_t)blockIdx.x * gstride : nullptr;
     unsigned char* incbase = lay.inc_in_smem ? smem_raw + lay.inc_off
@@ -1821,19 +1823,23 @@ __device__ __forceinline__ void cta_run(const KParams& p, unsigned char* smem_ra
     }
 }
 
-// Two CTAs per SM for the FP32 factors (the 157-species matrix is ~100 KB).
+// Two CTAs per SM for the FP32 factors (the 157-species matrix is ~100 KB) and
+// for RK2, whose registers would pass 128 otherwise (600 systems of 200 species:
+// 8.3 ms with one, 4.7 ms with two).
 #ifndef WIND_CTA_MIXED_BLOCKS
 #define WIND_CTA_MIXED_BLOCKS 2
 #endif
-template <int SOLVER>
+template <int METHOD, int SOLVER>
 struct CtaMinBlocks {
-    static constexpr int value = SOLVER == WIND_SOLVER_MIXED ? WIND_CTA_MIXED_BLOCKS : 1;
+    static constexpr int value = METHOD == WIND_METHOD_RK2          ? 2
+                                 : SOLVER == WIND_SOLVER_MIXED ? WIND_CTA_MIXED_BLOCKS
+                                                               : 1;
 };
 
 // TC = true: MIXED with the inverse's rank updates on the tensor cores
 // (the MIXED_TC solver).
 template <int METHOD, int CTRL, int SOLVER, bool TC = false>
-__global__ void __launch_bounds__(CTA_THREADS, CtaMinBlocks<SOLVER>::value)
+__global__ void __launch_bounds__(CTA_THREADS, CtaMinBlocks<METHOD, SOLVER>::value)
     k_cta(const KParams p, double* gscratch, size_t gstride, int smem_cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cta_run<METHOD, CTRL, SOLVER, TC>(p, smem_raw, gscratch, gstride, smem_cap);

@@ -85,7 +85,7 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
     const int threads = p.n_eq <= CTA_THREADS / 2 && !tc ? CTA_THREADS / 2 : CTA_THREADS;
     int caps[2] = {smem_optin(), 0};
     int ncap = 1;
-    if (solver == WIND_SOLVER_MIXED && CtaMinBlocks<WIND_SOLVER_MIXED>::value >= 2) caps[ncap++] = smem_half(fn);
+    if (solver == WIND_SOLVER_MIXED && CtaMinBlocks<WIND_METHOD_SIE, WIND_SOLVER_MIXED>::value >= 2) caps[ncap++] = smem_half(fn);
     // ranking: the matrix in shared memory first (a matrix in global memory
     // is read and written on every trailing update), then blocks per SM;
     // the batch can use; ties keep the larger budget
@@ -93,7 +93,8 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
     CtaPlan best{};
     int best_score = 0;
     for (int i = 0; i < ncap; i++) {
-        const CtaLayout lay(p.n_eq, p.n_react, p.linear != nullptr, solver, caps[i], tc);
+        const CtaLayout lay(p.n_eq, p.n_react, p.linear != nullptr, solver, caps[i], tc,
+                            o.method == WIND_METHOD_SIE);
         if (lay.bytes > caps[i]) continue;
         // the tensor-core staging must sit in shared memory, and the matrix
         // with it (the MMA operands are built from it every panel)
@@ -119,8 +120,8 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
     return WIND_OK;
 }
 
-size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int solver) {
-    const CtaLayout lay(n_eq, n_react, lin, solver, smem_optin());
+size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int method, int solver) {
+    const CtaLayout lay(n_eq, n_react, lin, solver, smem_optin(), false, method == WIND_METHOD_SIE);
     return lay.slot_doubles() * sizeof(double);
 }
 

@@ -51,7 +51,8 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
         // the solver each group runs (AUTO: MIXED above 32 species, LU_F64 below)
         const int gs = resolve_solver(solver, p.kind, p.n_eq);
         if (p.n_eq > 32) {
-            const CtaLayout lay(p.n_eq, p.n_react, p.linear != nullptr, gs, cap);
+            const CtaLayout lay(p.n_eq, p.n_react, p.linear != nullptr, gs, cap, false,
+                                o.method == WIND_METHOD_SIE);
             smem = std::max(smem, (size_t)lay.bytes);
             gslot = std::max(gslot, lay.slot_doubles());
             gneed = std::max(gneed, lay.g_doubles);

@@ -94,7 +94,7 @@ static size_t footprint(const ServerRequest& r, const wind_server_config& cfg) {
     if (r.kind == WIND_NET_MASS_ACTION && r.N > wind::WIND_TEAM_MAX_EQ) {
         const int solver = (cfg.method == WIND_METHOD_RK2) ? WIND_SOLVER_LU_F64
                                                              : wind::resolve_solver(cfg.solver, r.kind, r.N);
-        b += wind::cta_scratch_bytes_per_block(r.N, r.n_react, !r.linear.empty(), solver) *
+        b += wind::cta_scratch_bytes_per_block(r.N, r.n_react, !r.linear.empty(), cfg.method, solver) *
              (size_t)wind::device_sm_count() * 2;
     }
     return b;
