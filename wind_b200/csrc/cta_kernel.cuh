@@ -58,6 +58,28 @@ constexpr int CTA_REC_MAXR = 8192;  // reactions up to which a slot holds record
 constexpr int CTA_CONV = 14; // misc[] slot: refinement converged (0/1)
 constexpr int CTA_TCPAR = 15; // misc[] slot: phase parity of the tensor-core mbarrier
 
+// Threads of a k_cta block.  A small system leaves half of 256 threads without an
+// equation, and half the threads let more blocks onto an SM (registers), which
+// counts while there are more systems than SMs (`many`).  The Gauss-Jordan
+// elimination and the implicit solves' rank updates share N^2 elements out over
+// the block, whose size counts where they last.  128 against 256 threads, us:
+//   Gauss-Jordan  N = 48: 1 system 963, 778; 600 systems 2064, 3583
+//                 N = 64: 1 system 1691, 1226; 600 systems 5193, 5894
+//                 N = 80: 600 systems 16137, 9468; N = 128: 1 system 25781, 10354
+//   LU_F64        N = 48: 1 system 1251, 1266; 600 systems 3623, 5849
+//                 N = 128: 1 system 3656, 3563; 600 systems 17344, 16916
+//   MIXED         N = 33: 600 systems 2599, 2976; N = 80: 1188, 1138 and 3600, 4056
+//                 N = 128: 1 system 2308, 2171; 600 systems 7924, 7623
+//   RK2           N = 64: 1 system 823, 824; 600 systems 1858, 2483
+// The tensor-core staging is laid out for 256.
+__host__ __device__ constexpr int cta_block_threads(int n, int solver, bool rk2, bool tc, bool many) {
+    const int half = CTA_THREADS / 2;
+    if (tc || n > half) return CTA_THREADS;
+    if (rk2) return half;
+    if (solver == WIND_SOLVER_GJE_F64) return many && n <= 64 ? half : CTA_THREADS;
+    return n <= 64 || (many && solver == WIND_SOLVER_MIXED && n <= 112) ? half : CTA_THREADS;
+}
+
 // A warp's pivot candidate for one panel column: its best row's panel
 // entries and the reciprocal of the entry in the column.
 template <typename T>

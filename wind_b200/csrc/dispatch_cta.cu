@@ -79,10 +79,8 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
     const int solver = method_solver(o);
     const bool tc = o.method == WIND_METHOD_SIE && o.solver == WIND_SOLVER_MIXED_TC;
     CtaFn fn = cta_fn(o.method, o.controller, o.solver);
-    // up to 128 species: 128 threads (600 systems of 64 species: 71.9 ms, 72.6
-    // with 256).  Shared memory for four of those blocks per SM would push the
-    // reaction records out to L2: 113.6 ms.
-    const int threads = p.n_eq <= CTA_THREADS / 2 && !tc ? CTA_THREADS / 2 : CTA_THREADS;
+    const int threads =
+        cta_block_threads(p.n_eq, solver, o.method == WIND_METHOD_RK2, tc, p.nsys > device_sm_count());
     int caps[2] = {smem_optin(), 0};
     int ncap = 1;
     if (solver == WIND_SOLVER_MIXED && CtaMinBlocks<WIND_METHOD_SIE, WIND_SOLVER_MIXED>::value >= 2) caps[ncap++] = smem_half(fn);
