@@ -8,7 +8,7 @@
 
 namespace wind {
 
-using LuFn = void (*)(KParams, int);
+using LuFn = void (*)(KParams, int, int);
 
 // The kernel of a size: rows padded to a multiple of four columns, on a team of
 // 8, 16 or 32 lanes.  (Two rows per lane -- half the shared-memory reads per
@@ -63,25 +63,36 @@ wind_status launch_lu(const wind_options& o, const KParams& p, cudaStream_t stre
     const LuKernel k = lu_kernel(p.n_eq, o.controller);
     const LuFn fn = k.fn;
     const int lanes = k.lanes;
-    const LuLayout lay(k.cols, p.n_eq, p.n_react, lin);
-    int tpw = 0;
+    // The sorted Jacobian terms are half of what a reaction takes, and the faster
+    // path while two teams fit an SM with them.  A batch that would get one (above
+    // some 1,620 reactions) goes without, with three: 4,000 systems of 32 species
+    // and 1,900 reactions, 40 attempts each, 48.0 ms with the terms, 28.9 without;
+    // one attempt 4.7 and 2.0 ms.
+    int tpw = 0, sorted = 1;
     int64_t resident = 0;  // warps
-    for (int t = 1; t <= 32 / lanes; t *= 2) {
-        const size_t smem = (size_t)t * lay.bytes;
-        if (smem > 227 * 1024) break;
-        const int64_t r = (int64_t)lu_blocks_per_sm(fn, smem) * device_sm_count();
-        if (r * t >= resident * tpw && r > 0) {
-            resident = r;
-            tpw = t;
+    size_t bytes = 0;      // of a team
+    for (sorted = 1; sorted >= 0; sorted--) {
+        bytes = (size_t)LuLayout(k.cols, p.n_eq, p.n_react, lin, sorted != 0).bytes;
+        tpw = 0;
+        resident = 0;
+        for (int t = 1; t <= 32 / lanes; t *= 2) {
+            const size_t smem = (size_t)t * bytes;
+            if (smem > 227 * 1024) break;
+            const int64_t r = (int64_t)lu_blocks_per_sm(fn, smem) * device_sm_count();
+            if (r * t >= resident * tpw && r > 0) {
+                resident = r;
+                tpw = t;
+            }
+            if (resident * tpw >= p.nsys) break;
         }
-        if (resident * tpw >= p.nsys) break;
+        if (!sorted || resident * tpw >= p.nsys || resident * tpw > device_sm_count()) break;
     }
     if (tpw == 0) return WIND_ERR_UNSUPPORTED;
-    const size_t smem = (size_t)tpw * lay.bytes;
+    const size_t smem = (size_t)tpw * bytes;
     const int grid = (int)std::min<int64_t>((p.nsys + tpw - 1) / tpw, resident);
     if (allow_block_smem((const void*)fn) != cudaSuccess)
         return launch_status("k_lu shared-memory attribute");
-    fn<<<grid, 32, smem, stream>>>(p, tpw);
+    fn<<<grid, 32, smem, stream>>>(p, tpw, sorted);
     g_launches++;
     return launch_status("k_lu launch");
 }

@@ -65,7 +65,7 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
                     return WIND_ERR_UNSUPPORTED;
                 size_t bytes = (size_t)(MIXED_THREADS / nm) * WarpLayout(nm, p.n_react, plin, gs).bytes;
                 if (gs == WIND_SOLVER_LU_F64) {
-                    const LuLayout lay(nm, p.n_eq, p.n_react, plin);
+                    const LuLayout lay(nm, p.n_eq, p.n_react, plin, true);
                     bytes = (size_t)mixed_teams(nm, lay.bytes, cap) * lay.bytes;
                 }
                 smem = std::max(smem, bytes);

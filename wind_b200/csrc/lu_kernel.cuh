@@ -60,13 +60,13 @@ struct LuLayout {
     // byte offsets inside one team's slice
     int rates, inc_off, inc, term_off, term, lt, vb, rows, rows2, pb, bytes;
     __host__ __device__ static int align16(int x) { return (x + 15) & ~15; }
-    __host__ __device__ LuLayout(int cols, int n, int R, bool lin) {
+    __host__ __device__ LuLayout(int cols, int n, int R, bool lin, bool sorted) {
         int off = 0;
         rates = off; off = align16(off + (2 * R + 2) * 8);       // signed rates
         inc_off = off; off = align16(off + (n + 1) * 4);
         inc = off; off = align16(off + (4 * R + 3 * n + 4) * 4);  // and the word read ahead
-        term_off = off; off = align16(off + (n + 1) * 4);
-        term = off; off = align16(off + (8 * R + 3 * n + 4) * 4);
+        term_off = off; off = align16(off + (sorted ? (n + 1) * 4 : 0));
+        term = off; off = align16(off + (sorted ? (8 * R + 3 * n + 4) * 4 : 0));
         lt = off; off = align16(off + (lin ? n * n * 8 : 0));     // dense term, widened once
         vb = off; off = align16(off + (cols + 1) * 8);           // state, and a zero
         // Jacobian rows: at the accepted state, and at the half step -- of up
@@ -91,7 +91,7 @@ struct LuCtx {
     const int* inc_off;
     const uint32_t* inc;
     const int* term_off;
-    const uint32_t* term;
+    const uint32_t* term;  // null: the Jacobian is summed in place
     const double* LT;  // LT[k*N + r] = L[r][k], or null
     double* vb;
     double* rows;      // Jacobian rows in use
@@ -168,6 +168,28 @@ __device__ __forceinline__ void lu_jac_row(const Ctx& c, int r) {
             *reinterpret_cast<double*>(reinterpret_cast<char*>(row) + rx_second(q[u])) = acc;
             acc = (q[u] & RX_MARK) ? 0.0 : acc;
         }
+    }
+}
+
+// The same without the term list, which is half of what a reaction takes: an
+// entry's terms are added where they stand, in the same order (70 to 100 cycles a
+// term against 20 to 25 from the list).
+template <int COLS>
+__device__ __noinline__ void lu_jac_row_in_place(const double* rates, const uint32_t* inc, int cnt, const double* vb,
+                                                 double* row, uint32_t last) {
+#pragma unroll
+    for (int t = 0; t < COLS; t += 2) *reinterpret_cast<double2*>(row + t) = make_double2(0.0, 0.0);
+#pragma unroll 2
+    for (int e = 0; e < cnt; e++) {
+        const uint32_t q = inc[e];
+        // (padding and s = 0, from `last` on, go to the column beside the row)
+        const bool in = (q & 0x7ffffu) < last;
+        const uint32_t a = in ? rx_first(q) : 8u * COLS, b = in ? rx_second(q) : 8u * COLS;
+        const double ks = rx_rate(rates, q), va = rx_at(vb, a), vc = rx_at(vb, b);
+        double* pa = reinterpret_cast<double*>(reinterpret_cast<char*>(row) + a);
+        *pa = fma(ks, vc, *pa);
+        double* pb = reinterpret_cast<double*>(reinterpret_cast<char*>(row) + b);
+        *pb = fma(ks, va, *pb);
     }
 }
 
@@ -339,85 +361,140 @@ __device__ __noinline__ double lu_solve_exact(int l, int leader, int N, int tm, 
     return lu_solve<GUARD, true>(c, a, f);
 }
 
-// Stage system s: rates, the dense term transposed, the incidence lists and
-// the Jacobian terms.  A species index >= N marks the system BAD_INPUT
-// (returned) and nothing of it is read again.
-template <int L, int COLS>
-__device__ __forceinline__ bool lu_stage(const LuCtx<L, COLS>& c, const KParams& p, int64_t s, double* rates,
-                                         int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, double* LT) {
-    const int N = c.N, R = p.n_react, l = c.l;
-    const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * R;
+// Stage a system (rates `k_in`, reactions `sp`, dense term `Lg` or null) into its
+// team's slice: signed rates, the dense term transposed, the incidence lists and,
+// if `sorted`, the Jacobian terms.  A species index >= N marks it BAD_INPUT
+// (returned) and nothing of it is read again.  U: reactions in flight in a lane.
+//
+// What has no order (counts, rates) is done with a reaction per lane; a lane then
+// walks the list of its species once.  With a walk per column, behind two looks of
+// every lane at every reaction, one attempt of 4,000 systems of 32 species took
+// 5.3 ms with 1,000 reactions and 0.96 ms with 320; now 1.0 and 0.32 ms.
+template <int L, int COLS, int U>
+__device__ __forceinline__ bool lu_stage(unsigned mask, int l, int N, int R, const double* k_in, const uint2* sp,
+                                         const float* Lg, unsigned char* base, bool sorted) {
+    static_assert(COLS <= L, "a lane per species");
+    constexpr int LDR = LuCtx<L, COLS>::LDR;
+    const LuLayout lay(COLS, N, R, Lg != nullptr, sorted);
+    double* rates = reinterpret_cast<double*>(base + lay.rates);
+    int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
+    uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
+    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
+    uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
+    double* LT = reinterpret_cast<double*>(base + lay.lt);
+    double* rows = reinterpret_cast<double*>(base + lay.rows);
+    // `at`, in each species' Jacobian row: the terms of each column, counted, then
+    // where the column's next one goes
+    int* at = reinterpret_cast<int*>(rows + (l < N ? l : 0) * LDR);
+    if (l < N) {
+        inc_off[l + 1] = 0;
+#pragma unroll 1
+        for (int col = 0; col < N; col++) at[col] = 0;
+    }
+    __syncwarp(mask);
     bool bad = false;
+#pragma unroll U
     for (int r = l; r < R; r += L) {
-        const double k = p.rates[s * R + r];
+        const double k = __ldg(k_in + r);
         const uint2 q = __ldg(sp + r);
         // the reactants' s is -2 where they are one species that is not made
         // again, the products' +2 where they are one that is not consumed
         const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
         rates[2 * r] = (double)min(-1, stoich(a, a, b, cc, d)) * k;
         rates[2 * r + 1] = (double)max(1, stoich(cc, a, b, cc, d)) * k;
-        const unsigned nn = (unsigned)N;
-        bad = bad || (q.x & 0xffffu) >= nn || (q.x >> 16) >= nn || (q.y & 0xffffu) >= nn || (q.y >> 16) >= nn;
-    }
-    if (__any_sync(c.mask, bad)) return true;
-    for (int j = l; j < N; j += L) {
-        int cnt = 0, terms = 0;
-        for (int r = 0; r < R; r++) {
-            const uint2 q = __ldg(sp + r);
-            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
-            cnt += (a == j) | (b == j) | (cc == j) | (d == j);
-            terms += stoich(j, a, b, cc, d) ? 2 : 0;
+        if (max(max(a, b), max(cc, d)) >= N) {
+            bad = true;
+        } else {
+            auto count = [&](bool on, int j) {
+                if (!on) return;
+                atomicAdd(inc_off + 1 + j, 1);
+                if (sorted && stoich(j, a, b, cc, d)) {
+                    int* row = reinterpret_cast<int*>(rows + j * LDR);
+                    atomicAdd(row + a, 1);
+                    atomicAdd(row + b, 1);
+                }
+            };
+            count(true, a);
+            count(b != a, b);
+            count(cc != a && cc != b, cc);
+            count(d != a && d != b && d != cc, d);
         }
-        inc_off[j + 1] = (cnt + 3) & ~3;
-        term_off[j + 1] = (terms + 3) & ~3;
     }
-    __syncwarp(c.mask);
+    __syncwarp(mask);
+    if (__any_sync(mask, bad)) return true;
+    int terms = 0;
+    if (l < N) {
+#pragma unroll 1
+        for (int col = 0; col < N; col++) terms += at[col];
+    }
+    const int room = l < N ? (inc_off[l + 1] + 3) & ~3 : 0, term_room = (terms + 3) & ~3;
+    const int inc_end = rx_scan<L>(mask, l, room), term_end = rx_scan<L>(mask, l, term_room);
+    if (l < N) {
+        inc_off[l + 1] = inc_end;
+        if (sorted) term_off[l + 1] = term_end;
+    }
     if (l == 0) {
-        inc_off[0] = term_off[0] = 0;
-        for (int j = 0; j < N; j++) {
-            inc_off[j + 1] += inc_off[j];
-            term_off[j + 1] += term_off[j];
-        }
+        inc_off[0] = 0;
+        if (sorted) term_off[0] = 0;
         rates[2 * R] = 0.0;
         rates[2 * R + 1] = __longlong_as_double(0x7ff8000000000000ll);
-        c.vb[COLS] = 0.0;
+        reinterpret_cast<double*>(base + lay.vb)[COLS] = 0.0;
     }
-    __syncwarp(c.mask);
-    for (int j = l; j < N; j += L) {
-        int o = inc_off[j];
-        for (int r = 0; r < R; r++) {
-            const uint2 q = __ldg(sp + r);
-            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
-            if (a != j && b != j && cc != j && d != j) continue;
-            const int st = stoich(j, a, b, cc, d);
+    __syncwarp(mask);
+    uint32_t* mine = inc + inc_end - room;
+    const int cnt = rx_list<L>(mask, l, N, R, sp, reinterpret_cast<uint32_t*>(base + lay.pb), mine);
+    if (l < N) {
+        int t = term_end - term_room;
+        const int t_first = t;
+#pragma unroll 1
+        for (int col = 0; col < N; col++) {
+            const int n = at[col];
+            at[col] = t;
+            t += n;
+        }
+        uint2 next = cnt ? __ldg(sp + mine[0]) : make_uint2(0u, 0u);
+#pragma unroll 1
+        for (int e = 0; e < cnt; e++) {
+            const uint2 q = next;
+            const int r = (int)mine[e];
+            if (e + 1 < cnt) next = __ldg(sp + mine[e + 1]);
+            const int a = q.x & 0xffff, b = q.x >> 16;
+            const int st = stoich(l, a, b, (int)(q.y & 0xffff), (int)(q.y >> 16));
             int slot = st < 0 ? 2 * r : 2 * r + 1;
             if (st == 0) slot = finite64(rates[2 * r]) || finite64(rates[2 * r + 1]) ? 2 * R : 2 * R + 1;  // 0 * k
-            inc[o++] = rx_pack(slot, a, b);
-        }
-        // d w / d y_a = k y_b, then d w / d y_b = k y_a, per column in list order
-        const int e0 = inc_off[j];
-        int t = term_off[j];
-        for (int col = 0; col < N; col++) {
-            const int t0 = t;
-            for (int e = e0; e < o; e++) {
-                const uint32_t q = inc[e];
-                const int slot = (int)(q & 0x7ffffu) >> 3, a = (int)(rx_first(q) >> 3), b = (int)(rx_second(q) >> 3);
-                if (slot >= 2 * R) continue;
-                if (a == col) term[t++] = rx_pack(slot, b, col);
-                if (b == col) term[t++] = rx_pack(slot, a, col);
+            mine[e] = rx_pack(slot, a, b);
+            if (sorted && st) {
+                // d w / d y_a = k y_b, then d w / d y_b = k y_a, per column in list order
+                const int ta = at[a], tb = a == b ? ta + 1 : at[b];
+                at[a] = ta + 1;
+                at[b] = tb + 1;
+                term[ta] = rx_pack(slot, b, a);
+                term[tb] = rx_pack(slot, a, b);
             }
-            if (t > t0) term[t - 1] |= RX_MARK;
         }
         // padding: rate zero, the zero beside the state, the column beside the row
-        while (o < inc_off[j + 1]) inc[o++] = rx_pack(2 * R, COLS, COLS);
-        while (t < term_off[j + 1]) term[t++] = rx_pack(2 * R, COLS, COLS);
-        if (LT) {
-            const float* Lg = p.linear + s * (int64_t)N * N;
-            for (int k = 0; k < N; k++) LT[k * N + j] = Lg[j * N + k];
+#pragma unroll 1
+        for (int e = cnt; e < room; e++) mine[e] = rx_pack(2 * R, COLS, COLS);
+        if (sorted) {
+            for (int col = 0, t0 = t_first; col < N; t0 = at[col], col++)
+                if (at[col] > t0) term[at[col] - 1] |= RX_MARK;
+            while (t < term_end) term[t++] = rx_pack(2 * R, COLS, COLS);
+        }
+        if (Lg) {
+#pragma unroll 1
+            for (int k = 0; k < N; k++) LT[k * N + l] = Lg[l * N + k];
         }
     }
-    __syncwarp(c.mask);
+    __syncwarp(mask);
     return false;
+}
+
+// The same, out of line: its registers are not the solve's.  (k_mixed, whose
+// registers are those of the CTA kernels, has it inline.)
+template <int L, int COLS>
+__device__ __noinline__ bool lu_stage_apart(unsigned mask, int l, int N, int R, const double* k_in, const uint2* sp,
+                                            const float* Lg, unsigned char* base, bool sorted) {
+    return lu_stage<L, COLS, 4>(mask, l, N, R, k_in, sp, Lg, base, sorted);
 }
 
 // Warps per SM the registers are planned for.  8 (250 registers at 32 columns)
@@ -428,13 +505,14 @@ constexpr int LU_BLOCKS = 8;
 
 // The persistent team loop over one group's systems: the first `tpw` teams of
 // every warp (of the block's first `teams` teams) take tickets from the group's
-// queue until it is empty.  `smem_raw` holds `teams` team slices.
+// queue until it is empty.  `smem_raw` holds `teams` team slices, laid out with or
+// without the sorted Jacobian terms (GUARD: with).
 template <int L, int COLS, bool GUARD, int CTRL>
-__device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw, int teams, int tpw) {
+__device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw, int teams, int tpw, bool sorted) {
     using Ctx = LuCtx<L, COLS>;
     constexpr int CAP = Cap<WIND_METHOD_SIE, CTRL>::value;
     const bool lin = p.linear != nullptr;
-    const LuLayout lay(COLS, p.n_eq, p.n_react, lin);
+    const LuLayout lay(COLS, p.n_eq, p.n_react, lin, sorted);
     const int lane = threadIdx.x & 31;
     Ctx c;
     c.l = lane % L;
@@ -452,18 +530,12 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
     c.live = false;
     c.N = p.n_eq;
     unsigned char* base = smem_raw + team * lay.bytes;
-    double* rates = reinterpret_cast<double*>(base + lay.rates);
-    int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
-    uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
-    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
-    uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
-    double* LT = lin ? reinterpret_cast<double*>(base + lay.lt) : nullptr;
-    c.rates = rates;
-    c.inc_off = inc_off;
-    c.inc = inc;
-    c.term_off = term_off;
-    c.term = term;
-    c.LT = LT;
+    c.rates = reinterpret_cast<double*>(base + lay.rates);
+    c.inc_off = reinterpret_cast<int*>(base + lay.inc_off);
+    c.inc = reinterpret_cast<uint32_t*>(base + lay.inc);
+    c.term_off = reinterpret_cast<int*>(base + lay.term_off);
+    c.term = sorted ? reinterpret_cast<uint32_t*>(base + lay.term) : nullptr;
+    c.LT = lin ? reinterpret_cast<double*>(base + lay.lt) : nullptr;
     c.vb = reinterpret_cast<double*>(base + lay.vb);
     double* rows = reinterpret_cast<double*>(base + lay.rows);
     double* rows2 = reinterpret_cast<double*>(base + lay.rows2);
@@ -495,7 +567,11 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
                     phase = FULL;  // no system left: idle turns from here on
                     break;
                 }
-                stop = lu_stage(c, p, s, rates, inc_off, inc, term_off, term, LT);
+                const double* k = p.rates + s * p.n_react;
+                const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * p.n_react;
+                const float* Lg = lin ? p.linear + s * (int64_t)N * N : nullptr;
+                stop = GUARD ? lu_stage<L, COLS, 1>(c.mask, l, N, p.n_react, k, sp, Lg, base, true)
+                             : lu_stage_apart<L, COLS>(c.mask, l, N, p.n_react, k, sp, Lg, base, sorted);
                 st = stop ? WIND_SYS_BAD_INPUT : WIND_SYS_OK;
                 y = (l < N) ? p.y[s * N + l] : 0.0;
                 tnow = p.tnow;
@@ -557,7 +633,11 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
         }
         c.rows = second ? rows2 : rows;
         if (c.live && (second || !jy_ok)) {
-            if (l < N) lu_jac_row<Ctx, COLS>(c, l);
+            if (l < N) {
+                if (GUARD || c.term) lu_jac_row<Ctx, COLS>(c, l);
+                else lu_jac_row_in_place<COLS>(c.rates, c.inc + c.inc_off[l], c.inc_off[l + 1] - c.inc_off[l], c.vb,
+                                               c.rows + l * Ctx::LDR, 16u * p.n_react);
+            }
             jy_ok = !second || lay.rows2 != lay.rows;
         }
         double x;
@@ -604,9 +684,9 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
 }
 
 template <int L, int COLS, int CTRL>
-__global__ void __launch_bounds__(32, LU_BLOCKS) k_lu(const KParams p, int tpw) {
+__global__ void __launch_bounds__(32, LU_BLOCKS) k_lu(const KParams p, int tpw, int sorted) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    lu_run<L, COLS, false, CTRL>(p, smem_raw, tpw, tpw);
+    lu_run<L, COLS, false, CTRL>(p, smem_raw, tpw, tpw, sorted != 0);
 }
 
 }  // namespace wind

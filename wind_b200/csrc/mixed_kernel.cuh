@@ -36,8 +36,8 @@ __device__ __forceinline__ void mixed_team_run(const KParams& p, unsigned char* 
 template <int NMAX, int CTRL, int SOLVER>
 __device__ __forceinline__ void mixed_warp_run(const KParams& p, unsigned char* smem_raw, int smem_cap) {
     if constexpr (SOLVER == WIND_SOLVER_LU_F64) {
-        const LuLayout lay(NMAX, p.n_eq, p.n_react, p.linear != nullptr);
-        lu_run<NMAX, NMAX, true, CTRL>(p, smem_raw, mixed_teams(NMAX, lay.bytes, smem_cap), 32 / NMAX);
+        const LuLayout lay(NMAX, p.n_eq, p.n_react, p.linear != nullptr, true);
+        lu_run<NMAX, NMAX, true, CTRL>(p, smem_raw, mixed_teams(NMAX, lay.bytes, smem_cap), 32 / NMAX, true);
     } else {
         warp_run<NMAX, CTRL>(p, smem_raw);
     }

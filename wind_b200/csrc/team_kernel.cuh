@@ -363,83 +363,133 @@ __device__ __forceinline__ double team_gje_step(const TeamCtx<NMAX>& c, const do
     return out;
 }
 
-// Stage system s: signed rates, the dense term transposed, the unit lists and,
-// with JAC, the Jacobian terms.  A species index >= N marks the system BAD_INPUT
-// (returned) and nothing of it is read again.
+// Stage a system (rates `k`, reactions `sp`, dense term `Lg` or null) into its
+// team's slice: signed rates, the dense term transposed, the unit lists and, with
+// JAC, the Jacobian terms.  A species index >= N marks it BAD_INPUT (returned) and
+// nothing of it is read again.
 template <int NMAX, bool JAC>
-__device__ __forceinline__ bool team_stage(const TeamCtx<NMAX>& c, const KParams& p, int64_t s, double* rates,
-                                           int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, float* LT) {
-    const int N = c.N, R = p.n_react, l = c.l;
-    const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * R;
+__device__ __forceinline__ bool team_stage(unsigned mask, int l, int N, int R, const double* k_in, const uint2* sp,
+                                           const float* Lg, unsigned char* base) {
+    const TeamLayout lay(NMAX, R, Lg != nullptr, JAC);
+    double* rates = reinterpret_cast<double*>(base + lay.rates);
+    int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
+    uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
+    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
+    uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
+    float* LT = reinterpret_cast<float*>(base + lay.lt);
+    double* v = reinterpret_cast<double*>(base + lay.vec);
+    // `at` (in w, which no system uses yet), one row per species: the terms of each
+    // column, counted, then where the column's next one goes
+    constexpr int LDA = 2 * NMAX + 1;
+    int* counts = reinterpret_cast<int*>(base + lay.w);
+    int* at = counts + (l < N ? l : 0) * LDA;
+    if (l < N) {
+        inc_off[l + 1] = 0;  // units of species l, counted here
+        if (JAC) {
+#pragma unroll 1
+            for (int col = 0; col < N; col++) at[col] = 0;
+        }
+    }
+    team_sync(mask);
     bool bad = false;
     for (int r = l; r < R; r += NMAX) {
-        const double k = p.rates[s * R + r];
+        const double k = __ldg(k_in + r);
         rates[2 * r] = -k;
         rates[2 * r + 1] = k;
         const uint2 q = __ldg(sp + r);
-        const unsigned nn = (unsigned)N;
-        bad = bad || (q.x & 0xffffu) >= nn || (q.x >> 16) >= nn || (q.y & 0xffffu) >= nn || (q.y >> 16) >= nn;
-    }
-    if (__any_sync(c.mask, bad)) return true;
-    // units of species l in reaction (a, b -> cc, d): nn times -, then np times +
-    if (l < N) {
-        int cnt = 0;
-        for (int r = 0; r < R; r++) {
-            const uint2 q = __ldg(sp + r);
-            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
-            cnt += (a == l) + (b == l) + (cc == l) + (d == l);
+        const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+        if (max(max(a, b), max(cc, d)) >= N) {
+            bad = true;
+        } else {
+            auto count = [&](int j) {
+                atomicAdd(inc_off + 1 + j, 1);
+                if (JAC) {
+                    atomicAdd(counts + j * LDA + a, 1);
+                    atomicAdd(counts + j * LDA + b, 1);
+                }
+            };
+            count(a);
+            count(b);
+            count(cc);
+            count(d);
         }
-        inc_off[l + 1] = (cnt + 3) & ~3;
-        if (JAC) term_off[l + 1] = (2 * cnt + 3) & ~3;
     }
-    team_sync(c.mask);
+    team_sync(mask);
+    if (__any_sync(mask, bad)) return true;
+    // units of species l in reaction (a, b -> cc, d): nn times -, then np times +;
+    // two terms each
+    const int units = l < N ? inc_off[l + 1] : 0;
+    const int room = (units + 3) & ~3, term_room = JAC ? (2 * units + 3) & ~3 : 0;
+    const int inc_end = rx_scan<NMAX>(mask, l, room), term_end = rx_scan<NMAX>(mask, l, term_room);
+    if (l < N) {
+        inc_off[l + 1] = inc_end;
+        if (JAC) term_off[l + 1] = term_end;
+    }
     if (l == 0) {
         inc_off[0] = 0;
-        for (int j = 0; j < N; j++) inc_off[j + 1] += inc_off[j];
-        if (JAC) {
-            term_off[0] = 0;
-            for (int j = 0; j < N; j++) term_off[j + 1] += term_off[j];
-        }
+        if (JAC) term_off[0] = 0;
         rates[2 * R] = 0.0;
-        c.v[NMAX] = 0.0;
+        v[NMAX] = 0.0;
     }
-    team_sync(c.mask);
+    team_sync(mask);
+    uint32_t* mine = inc + inc_end - room;
+    int e = rx_list<NMAX>(mask, l, N, R, sp, reinterpret_cast<uint32_t*>(v + NMAX + 2), mine);
     if (l < N) {
-        int o = inc_off[l];
-        for (int r = 0; r < R; r++) {
-            const uint2 q = __ldg(sp + r);
-            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
-            const int nn = (a == l) + (b == l), np = (cc == l) + (d == l);
-            for (int u = 0; u < nn + np; u++) inc[o++] = rx_pack(2 * r + (u >= nn), a, b);
-        }
+        int t = term_end - term_room;
         if (JAC) {
+#pragma unroll 1
+            for (int col = 0; col < N; col++) {
+                t += at[col];
+                at[col] = t;  // where the column ends
+            }
+        }
+        // reactions to units and terms, from the end of the list (which only grows)
+        uint2 next = e ? __ldg(sp + mine[e - 1]) : make_uint2(0u, 0u);
+#pragma unroll 1
+        for (int o = units; e > 0;) {
+            const uint2 q = next;
+            const int r = (int)mine[--e];
+            if (e) next = __ldg(sp + mine[e - 1]);
+            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+            const int nn = (a == l) + (b == l), n = nn + (cc == l) + (d == l);
+            o -= n;
             // d w / d y_a = k y_b, then d w / d y_b = k y_a: per reaction all
             // units of the first before the second
-            int t = term_off[l];
-            for (int col = 0; col < N; col++) {
-                const int t0 = t;
-                for (int e = inc_off[l]; e < o;) {
-                    const uint32_t q = inc[e];
-                    const int r = (int)(q & 0x7ffffu) >> 4, a = (int)(rx_first(q) >> 3), b = (int)(rx_second(q) >> 3);
-                    int n = e + 1;  // the reaction's units are neighbours
-                    while (n < o && ((int)(inc[n] & 0x7ffffu) >> 4) == r) n++;
-                    if (a == col)
-                        for (int u = e; u < n; u++) term[t++] = rx_pack((int)(inc[u] & 0x7ffffu) >> 3, b, col);
-                    if (b == col)
-                        for (int u = e; u < n; u++) term[t++] = rx_pack((int)(inc[u] & 0x7ffffu) >> 3, a, col);
-                    e = n;
+            int ta = 0, tb = 0;
+            if (JAC) {
+                ta = at[a] - n;
+                tb = (a == b ? ta : at[b]) - n;
+                at[a] = ta;
+                at[b] = tb;
+                if (a == b) {
+                    const int first = tb;
+                    tb = ta;
+                    ta = first;
                 }
-                if (t > t0) term[t0] |= RX_MARK;
             }
-            while (t < term_off[l + 1]) term[t++] = rx_pack(2 * R, NMAX, NMAX) | RX_MARK;
+            for (int u = 0; u < n; u++) {
+                const int slot = 2 * r + (u >= nn);
+                mine[o + u] = rx_pack(slot, a, b);
+                if (JAC) {
+                    term[ta + u] = rx_pack(slot, b, a);
+                    term[tb + u] = rx_pack(slot, a, b);
+                }
+            }
         }
-        while (o < inc_off[l + 1]) inc[o++] = rx_pack(2 * R, NMAX, NMAX);
-        if (LT) {
-            const float* Lg = p.linear + s * (int64_t)N * N;
+        if (JAC) {
+            // (`at` is where the columns begin now)
+            for (int col = 0; col < N; col++) {
+                const int end = col + 1 < N ? at[col + 1] : t;
+                if (end > at[col]) term[at[col]] |= RX_MARK;
+            }
+            while (t < term_end) term[t++] = rx_pack(2 * R, NMAX, NMAX) | RX_MARK;
+        }
+        for (e = units; e < room; e++) mine[e] = rx_pack(2 * R, NMAX, NMAX);
+        if (Lg) {
             for (int k = 0; k < N; k++) LT[k * NMAX + l] = Lg[l * N + k];
         }
     }
-    team_sync(c.mask);
+    team_sync(mask);
     return false;
 }
 
@@ -465,18 +515,12 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
     c.w = reinterpret_cast<double*>(base + lay.w);
     c.v = reinterpret_cast<double*>(base + lay.vec);
     c.f = c.v + NMAX + 2;
-    float* LT = lin ? reinterpret_cast<float*>(base + lay.lt) : nullptr;
-    double* rates = reinterpret_cast<double*>(base + lay.rates);
-    int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
-    uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
-    c.LT = LT;
-    c.rates = rates;
-    c.inc_off = inc_off;
-    c.inc = inc;
-    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
-    uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
-    c.term_off = term_off;
-    c.term = term;
+    c.LT = lin ? reinterpret_cast<float*>(base + lay.lt) : nullptr;
+    c.rates = reinterpret_cast<double*>(base + lay.rates);
+    c.inc_off = reinterpret_cast<int*>(base + lay.inc_off);
+    c.inc = reinterpret_cast<uint32_t*>(base + lay.inc);
+    c.term_off = reinterpret_cast<int*>(base + lay.term_off);
+    c.term = reinterpret_cast<uint32_t*>(base + lay.term);
     const int N = c.N, l = c.l;
     const uint64_t t_start = p.timeout_ns ? global_ns() : 0;
     const double tend = p.tend;
@@ -499,7 +543,9 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
                 if (l == 0) ticket = atomicAdd(&p.counters[CNT_QUEUE], 1ull);
                 s = (int64_t)__shfl_sync(c.mask, ticket, c.leader);
                 if (s >= p.nsys) return;
-                stop = team_stage<NMAX, SIE>(c, p, s, rates, inc_off, inc, term_off, term, LT);
+                stop = team_stage<NMAX, SIE>(c.mask, l, N, p.n_react, p.rates + s * p.n_react,
+                                             reinterpret_cast<const uint2*>(p.species) + s * p.n_react,
+                                             lin ? p.linear + s * (int64_t)N * N : nullptr, base);
                 st = stop ? WIND_SYS_BAD_INPUT : WIND_SYS_OK;
                 y = (l < N) ? p.y[s * N + l] : 0.0;
                 tnow = p.tnow;
