@@ -33,58 +33,75 @@ void record_cuda_error(cudaError_t e, const char* where) {
 }
 const char* last_error_text() { return t_last_error; }
 
-// The current CUDA context, read through the driver entry point the runtime
-// hands out (no link against the driver library is needed).
-static CUcontext current_context() {
-    using GetCtx = CUresult (*)(CUcontext*);
-    static GetCtx fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<GetCtx>(f);
-    }();
+template <class Fn>
+static Fn driver_entry(const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
+        f = nullptr;
+    }
+    return reinterpret_cast<Fn>(f);
+}
+
+bool current_context(ContextKey* out) {
+    static const auto get = driver_entry<CUresult (*)(CUcontext*)>("cuCtxGetCurrent");
+    static const auto id = driver_entry<CUresult (*)(CUcontext, unsigned long long*)>("cuCtxGetId");
+    *out = ContextKey{};
     CUcontext c = nullptr;
-    if (!fn || fn(&c) != CUDA_SUCCESS) return nullptr;
-    return c;
+    if (!get || !id || get(&c) != CUDA_SUCCESS || !c || id(c, &out->id) != CUDA_SUCCESS) return false;
+    out->handle = c;
+    return true;
+}
+
+// The library's pool of the current device and context, or null (then the
+// device's default pool serves).
+static cudaMemPool_t library_pool() {
+    struct Pool {
+        int device;
+        ContextKey ctx;
+        cudaMemPool_t pool;
+    };
+    static std::mutex mu;
+    static std::vector<Pool> pools;
+    int dev = -1;
+    ContextKey ctx;
+    std::lock_guard<std::mutex> g(mu);
+    if (cudaGetDevice(&dev) != cudaSuccess || !current_context(&ctx)) return nullptr;
+    for (const Pool& e : pools)
+        if (e.device == dev && e.ctx.id == ctx.id) return e.pool;
+    // a context that took over a destroyed one's handle: its pool went with it
+    for (size_t i = 0; i < pools.size();) {
+        if (pools[i].device == dev && pools[i].ctx.handle == ctx.handle) pools.erase(pools.begin() + i);
+        else i++;
+    }
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t made = nullptr;
+    uint64_t keep = POOL_KEEP;
+    if (cudaMemPoolCreate(&made, &props) != cudaSuccess) return nullptr;
+    if (cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaMemPoolDestroy(made);
+        return nullptr;
+    }
+    pools.push_back({dev, ctx, made});
+    return made;
 }
 
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t stream) {
-    struct Pool {
-        cudaMemPool_t pool;
-        CUcontext ctx;  // made in this context; a device reset leaves another one
-    };
-    constexpr int MAX_DEVICES = 64;
-    static std::mutex mu;
-    static Pool pools[MAX_DEVICES] = {};
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    int dev = -1;
-    cudaMemPool_t pool = nullptr;
     // inside a capture the allocation is the graph's, not a pool's
-    if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-        cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < MAX_DEVICES) {
-        std::lock_guard<std::mutex> g(mu);
-        CUcontext ctx = current_context();
-        Pool& e = pools[dev];
-        if (!e.pool || e.ctx != ctx) {
-            e.pool = nullptr;
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.handleTypes = cudaMemHandleTypeNone;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            cudaMemPool_t made = nullptr;
-            uint64_t keep = POOL_KEEP;
-            if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
-                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
-                e.pool = made;
-                e.ctx = current_context();
-            }
+    if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        cudaMemPool_t pool = library_pool();
+        if (pool) {
+            if (cudaMallocFromPoolAsync(p, bytes, pool, stream) == cudaSuccess) return cudaSuccess;
+            // what the pool keeps unused goes back before the device's own pool is asked
+            (void)cudaMemPoolTrimTo(pool, 0);
         }
-        pool = e.pool;
     }
-    if (pool) return cudaMallocFromPoolAsync(p, bytes, pool, stream);
     (void)cudaGetLastError();
     return cudaMallocAsync(p, bytes, stream);
 }

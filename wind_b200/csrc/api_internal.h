@@ -96,10 +96,20 @@ inline bool device_ptr(const void* ptr) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// The current CUDA context (false: none, or the driver does not tell).  The id is
+// never used again, whereas a context made after a device reset may have the old
+// one's handle.
+struct ContextKey {
+    void* handle = nullptr;
+    unsigned long long id = 0;
+};
+bool current_context(ContextKey* out);
+
 // Stream-ordered device memory from the library's own pool of the current device
-// (api.cu).  The device's default pool gives everything back at every
+// and context (api.cu).  The device's default pool gives everything back at every
 // synchronisation, and a call after an idle moment then maps its memory again
-// (about 0.4 ms); this one keeps up to POOL_KEEP bytes.  Freed with
+// (about 0.4 ms); this one keeps up to POOL_KEEP bytes, gives them back when it
+// cannot serve a request, and leaves that request to the default pool.  Freed with
 // cudaFreeAsync; safe from any thread and on any stream.
 constexpr uint64_t POOL_KEEP = 64ull << 20;
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t stream);

@@ -36,8 +36,6 @@
 //    WIND_ERR_UNSUPPORTED before anything is cleared or launched, so no
 //    group's state has been touched and the call can be retried with the
 //    allocating entry point.
-#include <cuda.h>
-
 #include <mutex>
 #include <vector>
 
@@ -52,24 +50,7 @@ static __device__ __align__(256) unsigned long long g_noalloc_counters[kNoallocS
 
 std::mutex g_noalloc_mu;
 unsigned long long* g_noalloc_addr[kMaxDevices] = {};
-CUcontext g_noalloc_ctx[kMaxDevices] = {};
-
-// The current CUDA context, read through the driver entry point the runtime
-// hands out (no link against the driver library is needed).
-CUcontext current_context() {
-    using GetCtx = CUresult (*)(CUcontext*);
-    static GetCtx fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<GetCtx>(f);
-    }();
-    CUcontext c = nullptr;
-    if (!fn || fn(&c) != CUDA_SUCCESS) return nullptr;
-    return c;
-}
+unsigned long long g_noalloc_ctx[kMaxDevices] = {};  // id of the context the address is of
 
 // Device address of g_noalloc_counters on the current device, looked up with
 // the device current on the first call and again whenever the context changed.
@@ -78,14 +59,15 @@ wind_status noalloc_scratch(unsigned long long** out) {
     if (cudaGetDevice(&dev) != cudaSuccess) return WIND_ERR_CUDA;
     if (dev < 0 || dev >= kMaxDevices) return WIND_ERR_UNSUPPORTED;
     std::lock_guard<std::mutex> g(g_noalloc_mu);
-    const CUcontext ctx = current_context();
-    if (!g_noalloc_addr[dev] || ctx != g_noalloc_ctx[dev]) {
+    wind::ContextKey ctx;
+    if (!wind::current_context(&ctx) || !g_noalloc_addr[dev] || ctx.id != g_noalloc_ctx[dev]) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_counters);
         if (e != cudaSuccess || !p) return wind::cuda_status(e != cudaSuccess ? e : cudaErrorInvalidSymbol,
                                                              "noalloc scratch address");
         g_noalloc_addr[dev] = static_cast<unsigned long long*>(p);
-        g_noalloc_ctx[dev] = current_context();
+        // (the lookup made the context if there was none)
+        g_noalloc_ctx[dev] = wind::current_context(&ctx) ? ctx.id : 0;
     }
     *out = g_noalloc_addr[dev];
     return WIND_OK;
