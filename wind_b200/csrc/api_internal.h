@@ -55,10 +55,10 @@ struct CtaPlan {
 };
 wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global, CtaPlan* out);
 wind_status launch_cta(const CtaPlan& pl, const KParams& p, cudaStream_t stream, double* scratch);
-// Global scratch (bytes) one resident CTA-kernel block needs for an N > 32
-// mass-action system with the full shared-memory budget (0 when everything
-// fits in shared memory).
-size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int method, int solver);
+// Global scratch (bytes) one resident CTA-kernel block cannot do without for an
+// N > 32 mass-action system with the full shared-memory budget (0 when everything
+// fits in shared memory; reaction records are not counted).
+size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int solver);
 extern std::atomic<int64_t> g_launches;
 // Largest N any kernel family accepts (lane/team kernels up to 32, CTA
 // kernels up to 256).
@@ -245,6 +245,8 @@ struct IntegrateCall {
 }  // namespace wind
 
 namespace wind {
+// `spare`: bytes of device scratch the launch may take beyond what it cannot do
+// without (reaction records of the N > 32 groups); `taken` gets what it took of them.
 wind_status launch_batch(const wind_options& o, const wind_group* groups, int ngroups,
-                         cudaStream_t stream);
+                         cudaStream_t stream, size_t spare = SIZE_MAX, size_t* taken = nullptr);
 }

@@ -10,7 +10,8 @@
 
 namespace wind {
 
-wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, cudaStream_t stream);
+wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, cudaStream_t stream, size_t spare,
+                         size_t* taken);
 
 // Streams and events for the builtin groups that run beside the mass-action
 // launch, kept per host thread and device and reused by every call (a
@@ -52,7 +53,8 @@ static wind_status fork_pool(size_t n, ForkPool** out) {
 }
 
 wind_status launch_batch(const wind_options& o, const wind_group* groups, int ngroups,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, size_t spare, size_t* taken) {
+    if (taken) *taken = 0;
     if (o.solver == WIND_SOLVER_MIXED_TC) return WIND_ERR_UNSUPPORTED;
     for (int g = 0; g < ngroups; g++) {
         wind_status st = check_network(&groups[g].net, groups[g].nsys);
@@ -109,7 +111,7 @@ wind_status launch_batch(const wind_options& o, const wind_group* groups, int ng
         st = launch_integrate(o, builtin[g], fp->streams[g]);
         cudaEventRecord(fp->done[g], fp->streams[g]);
     }
-    if (st == WIND_OK) st = launch_mixed(o, mass, stream);
+    if (st == WIND_OK) st = launch_mixed(o, mass, stream, spare, taken);
     if (fp)
         for (size_t g = 0; g < builtin.size(); g++) cudaStreamWaitEvent(stream, fp->done[g], 0);
     cudaFreeAsync(counters, stream);

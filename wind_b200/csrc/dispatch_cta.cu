@@ -118,9 +118,9 @@ wind_status plan_cta(const wind_options& o, const KParams& p, bool allow_global,
     return WIND_OK;
 }
 
-size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int method, int solver) {
-    const CtaLayout lay(n_eq, n_react, lin, solver, smem_optin(), false, method == WIND_METHOD_SIE);
-    return lay.slot_doubles() * sizeof(double);
+size_t cta_scratch_bytes_per_block(int n_eq, int n_react, bool lin, int solver) {
+    const CtaLayout lay(n_eq, n_react, lin, solver, smem_optin());
+    return lay.g_doubles * sizeof(double);
 }
 
 wind_status launch_cta(const CtaPlan& pl, const KParams& p, cudaStream_t stream, double* scratch) {

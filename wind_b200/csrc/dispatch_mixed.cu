@@ -38,8 +38,9 @@ bool team_admitted(int n, int R, bool lin, bool lists, int teams, size_t budget)
 bool warp_admitted(int n, int R, bool lin, int solver, int threads, size_t budget);
 
 // Launch all mass-action groups `ps` (kernel parameters with their counters
-// already set) in one kernel on `stream`.
-wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, cudaStream_t stream) {
+// already set) in one kernel on `stream`.  `spare`, `taken`: as launch_batch.
+wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, cudaStream_t stream, size_t spare,
+                         size_t* taken) {
     if (ps.empty()) return WIND_OK;
     const int solver = (o.method == WIND_METHOD_RK2) ? WIND_SOLVER_LU_F64 : o.solver;
     int dev = 0, cap = 227 * 1024;
@@ -97,6 +98,7 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
     unsigned char* dparams = nullptr;
     if (pool_alloc((void**)&dparams, pbytes + obytes + 16, stream) != cudaSuccess) return WIND_ERR_NOMEM;
     double* gscratch = nullptr;
+    if ((gslot - gneed) * grid * sizeof(double) > spare) gslot = gneed;
     if (gslot && pool_alloc((void**)&gscratch, gslot * grid * sizeof(double), stream) != cudaSuccess) {
         (void)cudaGetLastError();
         gscratch = nullptr;
@@ -121,6 +123,7 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
                                                   (int)ps.size(), gscratch, gslot, cap);
         g_launches++;
         st = launch_status("k_mixed launch");
+        if (taken) *taken = (gslot - gneed) * grid * sizeof(double);
     }
     cudaFreeAsync(dparams, stream);
     if (gscratch) cudaFreeAsync(gscratch, stream);

@@ -62,6 +62,7 @@ struct Slot {
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     std::vector<ServerRequest*> reqs;
+    size_t extra = 0;  // device bytes of its launch beyond the requests' footprints
     bool busy = false;
 };
 
@@ -87,14 +88,16 @@ struct Server {
 // global scratch the CTA kernels take for what does not fit in shared
 // memory (one slot per resident block: up to two blocks per SM), counted
 // in full for every such request since each launch sizes it for its
-// largest group.
+// largest group.  (Reaction records, which a launch can do without, are not in
+// it: a launch takes them while half of the budget is free beside them, and they
+// count as resident until it is done.)
 static size_t footprint(const ServerRequest& r, const wind_server_config& cfg) {
     size_t b = r.nsys * (size_t)r.N * 8 + r.constants.size() * 8 + r.rates.size() * 8 +
                r.species.size() * 2 + r.linear.size() * 4 + r.nsys * 12 + 64 * 8;
     if (r.kind == WIND_NET_MASS_ACTION && r.N > wind::WIND_TEAM_MAX_EQ) {
         const int solver = (cfg.method == WIND_METHOD_RK2) ? WIND_SOLVER_LU_F64
                                                              : wind::resolve_solver(cfg.solver, r.kind, r.N);
-        b += wind::cta_scratch_bytes_per_block(r.N, r.n_react, !r.linear.empty(), cfg.method, solver) *
+        b += wind::cta_scratch_bytes_per_block(r.N, r.n_react, !r.linear.empty(), solver) *
              (size_t)wind::device_sm_count() * 2;
     }
     return b;
@@ -170,6 +173,7 @@ static void worker_main(Server* S) {
     while (true) {
         std::vector<ServerRequest*> batch;
         Slot* slot = nullptr;
+        size_t spare = 0;
         {
             std::unique_lock<std::mutex> lk(S->mu);
             // admission by device footprint, in arrival order
@@ -196,6 +200,8 @@ static void worker_main(Server* S) {
                 }
                 slot->busy = true;
                 slot->reqs = batch;
+                const size_t half = (size_t)S->cfg.hbm_budget_bytes / 2;
+                spare = half > S->resident ? half - S->resident : 0;
             } else {
                 bool any_busy = false;
                 for (Slot& sl : S->slots) any_busy |= sl.busy;
@@ -212,7 +218,8 @@ static void worker_main(Server* S) {
                 if (st == WIND_OK) st = upload(*r, slot->stream);
                 groups.push_back(group_of(*r));
             }
-            if (st == WIND_OK) st = launch_batch(o, groups.data(), (int)groups.size(), slot->stream);
+            size_t extra = 0;
+            if (st == WIND_OK) st = launch_batch(o, groups.data(), (int)groups.size(), slot->stream, spare, &extra);
             for (ServerRequest* r : batch) {
                 if (st != WIND_OK) break;
                 cudaMemcpyAsync(r->h_y, r->d_y, r->nsys * (size_t)r->N * 8, cudaMemcpyDeviceToHost, slot->stream);
@@ -222,6 +229,8 @@ static void worker_main(Server* S) {
             for (ServerRequest* r : batch) r->result = st;
             cudaEventRecord(slot->done, slot->stream);
             std::lock_guard<std::mutex> lk(S->mu);
+            slot->extra = extra;
+            S->resident += extra;
             S->launches++;
         }
         // completion of in-flight batches
@@ -240,6 +249,8 @@ static void worker_main(Server* S) {
                 S->completed++;
                 S->systems_done += r->nsys;
             }
+            S->resident -= sl.extra;
+            sl.extra = 0;
             sl.reqs.clear();
             sl.busy = false;
             S->cv_done.notify_all();
