@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "api_internal.h"
+#include "float32.h"
 #include "networks.cuh"
 
 using namespace wind;

@@ -26,6 +26,7 @@
 
 #include "../../include/wind.h"
 #include "../../include/wind_legacy.h"
+#include "float32.h"
 
 #ifndef WIND_LEGACY_NET
 #error "WIND_LEGACY_NET must name the network (WIND_NET_*)"
@@ -33,11 +34,6 @@
 #ifndef WIND_LEGACY_METHOD
 #error "WIND_LEGACY_METHOD must be WIND_METHOD_SIE or WIND_METHOD_RK2"
 #endif
-
-// libwind's integration of float32 host arrays (api.cu), in place on y.
-extern "C" int wind_integrate_f32(const wind_options* opt, int32_t kind, int32_t n_eq, int32_t n_const, double tnow,
-                                  double tend, int32_t n_integration_steps, const float* constants, float* y,
-                                  int64_t nsys, double atol, double rtol, int64_t* total_nsteps);
 
 static int legacy_n_const(int kind) {
     return kind == WIND_NET_KATZ96 ? 10 : (kind == WIND_NET_NR_TEST ? 4 : 2);
