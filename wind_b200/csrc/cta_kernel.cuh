@@ -1,12 +1,13 @@
 // cta_kernel.cuh -- persistent CTA-per-system integrator for mass-action
 // networks with 32 < N <= 256 (the 64- and 157-species classes).
 //
-// One CTA (256 threads) integrates one system at a time and pulls the next
-// ticket from the device work queue when it finishes.  Thread l owns
-// equation l (N <= 256): its y, y1, y2 live in registers.  Per system the CTA
+// One CTA (128 or 256 threads, cta_block_threads) integrates one system at a time
+// and pulls the next ticket from the device work queue when it finishes.  Thread l
+// owns equation l (N <= 256): its y, y1, y2 live in registers.  Per system the CTA
 // builds per-species incidence lists of the reactions (CSR, reaction ids
-// ascending), so thread j evaluates f_j and row j of the Jacobian from the
-// ~4R/N reactions that touch species j instead of all R.
+// ascending) and, for the implicit solves, records of them where a launch has the
+// room (cta_incidences), so thread j evaluates f_j and row j of the Jacobian from
+// the ~4R/N reactions that touch species j instead of all R.
 //
 // Solvers (selected at compile time):
 //  GJE_F64  the reference's unpivoted Gauss-Jordan inverse, reference
@@ -15,14 +16,17 @@
 //  LU_F64   blocked right-looking LU with partial pivoting, FP64, on the
 //           matrix [A | b] in shared memory (global scratch when it does not
 //           fit), followed by blocked triangular solves;
-//  MIXED    FP32 factors without pivoting, FP64 residual r = f - (x - h J x)
-//           evaluated from the reactions (no FP64 matrix), FP64 refinement
-//           until the correction is below 1e-6 of |x| (per 32-row slice; at
-//           most two steps), else the substep is redone with partial
-//           pivoting.  Its footprint lets two CTAs share an SM at N = 157.
+//  MIXED    one FP32 Gauss-Jordan inverse per attempt, unpivoted and blocked
+//           (cta_gj_invert) or, at step sizes where that one failed, pivoted
+//           (cta_gj_invert_pivoted); every solve of the attempt refines around it
+//           in FP64 with the residual r = f - (x - h J x) from the reactions, no
+//           FP64 matrix, until the predicted error is below 2^-33 of |x|
+//           (cta_refine).  What does not refine goes to an FP32 LU with partial
+//           pivoting (cta_mixed_pivoted_solve).  Its footprint lets two CTAs
+//           share an SM at N = 157.
 //
-// Blocked LU (panel width CTA_NB = 16).  Rows never move: logical row i is
-// physical row piv[i].  For each panel (cta_lu, partial pivoting):
+// Blocked LU (cta_lu, panel width CTA_NB = 16).  Rows never move: logical row i is
+// physical row piv[i].  For each panel:
 //  1. panel factorisation: thread p holds the 16 panel entries of physical
 //     row p in registers.  Per column one CTA barrier: each warp's best
 //     candidate (max |a| by a __reduce_max_sync key) publishes its row's
@@ -34,9 +38,6 @@
 //  3. U12 = L11^-1 A12 for the 16 pivot rows, one thread per column;
 //  4. trailing update A22 -= L21 U12 over act[] x columns, 4x4 register
 //     tiles with 16-byte shared-memory vectors.
-// The MIXED solver factors without pivoting (cta_lu_nopiv): warp 0 factors
-// the 16x16 diagonal block with shuffles, the rows below form their own
-// multipliers, then steps 3 and 4 -- three barriers per panel.
 // The right-hand side is column N, so the forward elimination comes with the
 // factorisation; the row stride is padded so that rows start 16 bytes apart
 // in the bank space (no conflicts when 32 rows are read at one column).
@@ -453,10 +454,9 @@ __device__ __forceinline__ void cta_u12(T* A, int k0, const int (&prow)[CTA_NB])
     }
 }
 
-// Trailing update A22 -= L21 U12 of the panel at k0: the active rows
-// (act[0..m) with pivoting, rows c0..N-1 in order without) times columns
-// c0..N, 4x4 register tiles with 16-byte vectors.
-template <typename T, bool NATURAL>
+// Trailing update A22 -= L21 U12 of the panel at k0: the active rows act[0..m)
+// times columns c0..N, 4x4 register tiles with 16-byte vectors.
+template <typename T>
 __device__ __forceinline__ void cta_trailing(T* A, int k0, const int (&prow)[CTA_NB]) {
     const CtaCtx& c = cta_ctx;
     constexpr int TR = 4;
@@ -469,7 +469,7 @@ __device__ __forceinline__ void cta_trailing(T* A, int k0, const int (&prow)[CTA
 #pragma unroll
         for (int r = 0; r < TR; r++) {
             const int rr = TR * ti + r;
-            rows[r] = rr < m ? (NATURAL ? c0 + rr : c.act[rr]) * ld : -1;
+            rows[r] = rr < m ? c.act[rr] * ld : -1;
         }
         T acc[TR][4];
 #pragma unroll
@@ -584,79 +584,7 @@ __device__ void cta_lu(T* A) {
         cta_u12<T>(A, k0, prow);
         __syncthreads();
         // 4. trailing update over act[0..m) x [c0, N]
-        cta_trailing<T, false>(A, k0, prow);
-        __syncthreads();
-    }
-}
-
-// LU without pivoting (the elimination order of the reference's
-// Gauss-Jordan inverse), for the FP32 factors of MIXED, whose refinement
-// checks convergence and falls back to cta_lu.  Per panel at k0: warp 0
-// factors the 16 x 16 diagonal block with shuffles; every row below then
-// computes its own multipliers in registers from U11 while the U12 columns
-// are formed; then the trailing update -- three barriers per panel against
-// nineteen with the pivot vote.
-template <typename T>
-__device__ void cta_lu_nopiv(T* A) {
-    const CtaCtx& c = cta_ctx;
-    const int N = c.N, tid = (int)threadIdx.x, ld = c.ld;
-    if (tid < N) c.piv[tid] = tid;
-    for (int k0 = 0; k0 < N; k0 += CTA_NB) {
-        const int kb = min(CTA_NB, N - k0);
-        if (tid < 32) {
-            const int lane = tid;
-            const bool mine = lane < kb;
-            T* row = A + (size_t)(k0 + (mine ? lane : 0)) * ld + k0;
-            T a[CTA_NB];
-#pragma unroll
-            for (int q = 0; q < CTA_NB / 4; q++) {
-                if (mine) ld4at(row + 4 * q, a + 4 * q);
-                else a[4 * q] = a[4 * q + 1] = a[4 * q + 2] = a[4 * q + 3] = (T)0;
-            }
-#pragma unroll
-            for (int j = 0; j < CTA_NB; j++) {
-                if (j < kb) {
-                    const T ri = __shfl_sync(0xffffffffu, nr_rcp(a[j]), j);
-                    if (lane == j) c.rinv[k0 + j] = (double)ri;
-                    const bool upd = mine && lane > j;
-                    const T l = a[j] * ri;
-                    if (upd) a[j] = l;
-#pragma unroll
-                    for (int jj = j + 1; jj < CTA_NB; jj++) {
-                        const T pv = __shfl_sync(0xffffffffu, a[jj], j);
-                        if (upd) a[jj] = fma(-l, pv, a[jj]);
-                    }
-                }
-            }
-            if (mine) {
-#pragma unroll
-                for (int q = 0; q < CTA_NB / 4; q++) st4at(row + 4 * q, a + 4 * q);
-            }
-        }
-        __syncthreads();
-        const int c0 = k0 + CTA_NB;
-        if (c0 > N) break;  // last panel: b was eliminated with the block
-        int prow[CTA_NB];
-#pragma unroll
-        for (int j = 0; j < CTA_NB; j++) prow[j] = (k0 + j) * ld;
-        if (tid >= c0 && tid < N) {
-            T* row = A + (size_t)tid * ld + k0;
-            T a[CTA_NB];
-#pragma unroll
-            for (int q = 0; q < CTA_NB / 4; q++) ld4at(row + 4 * q, a + 4 * q);
-#pragma unroll
-            for (int j = 0; j < CTA_NB; j++) {
-                const T l = a[j] * (T)c.rinv[k0 + j];
-                a[j] = l;
-#pragma unroll
-                for (int jj = j + 1; jj < CTA_NB; jj++) a[jj] = fma(-l, A[prow[j] + k0 + jj], a[jj]);
-            }
-#pragma unroll
-            for (int q = 0; q < CTA_NB / 4; q++) st4at(row + 4 * q, a + 4 * q);
-        }
-        cta_u12<T>(A, k0, prow);
-        __syncthreads();
-        cta_trailing<T, true>(A, k0, prow);
+        cta_trailing<T>(A, k0, prow);
         __syncthreads();
     }
 }
@@ -1445,10 +1373,11 @@ __device__ void cta_gje_exact(double h, double* M, double* Inv) {
     __syncthreads();
 }
 
-// One substep of size h on c.v (in place).  Returns true when the MIXED
-// solve had to be redone with pivoting (uniform across the CTA).
+// One substep of size h on c.v (in place): RK2, or SIE with an FP64 solve (MIXED
+// works attempt by attempt, in cta_run).
 template <int METHOD, int CTRL, int SOLVER>
-__device__ bool cta_substep(double h, void* mat, double* gM, int cnt) {
+__device__ void cta_substep(double h, void* mat, double* gM, int cnt) {
+    static_assert(METHOD == WIND_METHOD_RK2 || SOLVER != WIND_SOLVER_MIXED, "MIXED has its own attempt");
     const CtaCtx& c = cta_ctx;
     const int N = c.N, tid = (int)threadIdx.x;
     const bool own = tid < N;
@@ -1456,42 +1385,19 @@ __device__ bool cta_substep(double h, void* mat, double* gM, int cnt) {
         cta_rhs();
         if (own) c.v[tid] = (xd(c.v[tid]) + xd(h) * xd(c.f[tid])).v;
         __syncthreads();
-        return false;
+        return;
     }
     if (SOLVER == WIND_SOLVER_GJE_F64) {
         cta_rhs();
         cta_gje_exact<CTRL>(h, gM, gM + (size_t)N * N);
-        return false;
+        return;
     }
-    using T = typename std::conditional<SOLVER == WIND_SOLVER_MIXED, float, double>::type;
-    T* A = static_cast<T*>(mat);
-    bool fell = false;
-    cta_build<T, false>(h, A, cnt);
-    if (SOLVER == WIND_SOLVER_MIXED) {
-        // unpivoted FP32 factors and up to two FP64 refinement steps (the
-        // second only when the first correction is not yet small); if the
-        // last correction is not small, redo the substep with pivoting
-        for (int pass = 0; pass < 2; pass++) {
-            if (pass == 0) cta_lu_nopiv<T>(A);
-            else cta_lu<T>(A);
-            cta_solve<T, false>(A);
-            for (int it = 0; it < 2; it++) {
-                if (own) c.r[tid] = c.f[tid] - (c.x[tid] - h * cta_jx(tid, c.x, cnt));
-                __syncthreads();
-                cta_solve<T, true>(A);
-                if (c.misc[CTA_CONV]) break;
-            }
-            if (c.misc[CTA_CONV] || pass == 1) break;
-            fell = true;
-            cta_build<T, false>(h, A, cnt);
-        }
-    } else {
-        cta_lu<T>(A);
-        cta_solve<T, false>(A);
-    }
+    double* A = static_cast<double*>(mat);
+    cta_build<double, false>(h, A, cnt);
+    cta_lu<double>(A);
+    cta_solve<double, false>(A);
     if (own) c.v[tid] = c.v[tid] + h * c.x[tid];
     __syncthreads();
-    return fell;
 }
 
 // The persistent CTA loop over one group's systems (blockDim.x a multiple of
@@ -1796,7 +1702,7 @@ __device__ __forceinline__ void cta_run(const KParams& p, unsigned char* smem_ra
                 }
                 for (int k = 0; k < nsub; k++) {
                     if (CTRL == WIND_CTRL_DEVICE) hs = fmin(t1 - t, hs);
-                    if (cta_substep<METHOD, CTRL, SOLVER>(hs, mat, gM, rec_cnt)) st |= WIND_SYS_REFINE_FALLBACK;
+                    cta_substep<METHOD, CTRL, SOLVER>(hs, mat, gM, rec_cnt);
                     t += hs;
                     if (pass == 1 && k == 0) {
                         vh_keep = own ? c.v[tid] : 0.0;
