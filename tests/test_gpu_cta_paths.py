@@ -51,3 +51,16 @@ def test_cta_mixed_large_steps(cuda_device, n):
     _, st, _ = lib.integrate(net, y_g, 0.0, 1.0, 1e-3, 1e-2, "sie", "mixed", "gold")
     assert (st & 8).any()
     assert mixed_err(y_g, y_l, 1e-3) <= 1e-5
+
+
+@pytest.mark.parametrize("solver,n", [("mixed", 157), ("lu_f64", 128)])
+def test_cta_launch_without_scratch(cuda_device, solver, n):
+    """Networks whose records do not fit shared memory, through the entry point
+    that allocates nothing (species lists) and the one that does (records in
+    scratch): the same terms in the same order, so the same bits."""
+    net, y0 = _net(n, 3, 10 * n)
+    wl = [W.Workload(net, y0, 0.0, 1e-5, 1e-4, 1e-3)]
+    (want, st, steps), = lib.integrate_batch(wl, "sie", solver, "gold")
+    (got, s, c), = lib.integrate_batch(wl, "sie", solver, "gold", noalloc=True)
+    assert steps.min() > 0
+    assert np.array_equal(got, want) and np.array_equal(s, st) and np.array_equal(c, steps)
