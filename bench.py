@@ -676,8 +676,8 @@ def katz96_extra(args, torch, dev, lib, _capi, C):
             drop[solver] = {"systems_per_s": net.nsys / statistics.median(ts)}
         os.environ.pop("WIND_LEGACY_SOLVER", None)
         drop["call"] = ("_Z19cudaIntegrateSystemffiPfS_iiff from lib/katz96/sie.so, pageable "
-                        "float32 host arrays, wall clock per call (host conversions, copies and "
-                        "the integration)")
+                        "float32 host arrays, wall clock per call (copies, conversions on the "
+                        "device and the integration)")
         out["e2e_dropin"] = drop
     except Exception as exc:  # the headline line must still print
         os.environ.pop("WIND_LEGACY_SOLVER", None)

@@ -1401,8 +1401,9 @@ __device__ void cta_substep(double h, void* mat, double* gM, int cnt) {
 }
 
 // The persistent CTA loop over one group's systems (blockDim.x a multiple of
-// 32, at least N and at least 64; CTA_THREADS with TC).  `gscratch` holds one slot of `gstride` >=
-// CtaLayout::g_doubles doubles per block (null when the layout needs none).
+// 32, at least N and at least 64; CTA_THREADS with TC).  `gscratch` holds one slot
+// of `gstride` >= CtaLayout::g_doubles doubles per block (null when the layout
+// needs none).
 template <int METHOD, int CTRL, int SOLVER, bool TC>
 __device__ __forceinline__ void cta_run(const KParams& p, unsigned char* smem_raw, double* gscratch,
                                         size_t gstride, int smem_cap) {

@@ -31,15 +31,16 @@
 // ascending) and, for the Jacobian, their terms sorted by column, so a row
 // entry is summed in a register, in the order of the unsorted list, and
 // stored without being read back.  Lists are padded to whole 16-byte words of
-// four with entries that add zero.
+// four with entries that add zero.  (With many reactions the terms cost resident
+// teams, and a launch may leave them out: lu_jac_row_in_place.)
 //
 // The dense term is widened to FP64 when a system is staged: a substep reads
 // each entry twice, and a conversion takes 12 to 24 cycles of a unit that the
 // pivot keys and reciprocals need too.  3,000 dense systems of 32 species and
-// 64 reactions: 704 to 637 ms (893 before this kernel).  The 4 KB a team that this costs take teams
-// away where there are many reactions, and the gain is smaller there: at looser
-// tolerances 68.3 to 62.0 ms with 64 reactions, 79.6 to 76.0 ms with 160, 92.7
-// to 91.3 ms with 240.
+// 64 reactions: 704 to 637 ms (893 before this kernel).  The 4 KB a team that this
+// costs take teams away where there are many reactions, and the gain is smaller
+// there: at looser tolerances 68.3 to 62.0 ms with 64 reactions, 79.6 to 76.0 ms
+// with 160, 92.7 to 91.3 ms with 240.
 //
 // The values are those of the one-row-per-lane kernel this replaced, bit for
 // bit: the same pivots, multipliers and order of every sum.

@@ -133,11 +133,12 @@ __device__ __forceinline__ void lu_solve_reg(const T (&A)[N * N], const T (&rinv
 // multiplier, a quotient 0/s or a product with a zero leaves every in-block
 // value as it is while nothing is infinite or NaN.  The block forms do the
 // in-block operations only, in the same order, so their results are the
-// full-width ones bit for bit (a zero's sign aside) whenever `max_hi` of the
-// values named below stays under HI_INF; otherwise the caller repeats the
-// substep full width.  A Katz96 substep then takes 12 divisions and 22
-// multiplications and subtractions in the Gauss-Jordan inverse instead of 50
-// and 1000, and one pivot comparison per column in the LU.
+// full-width ones bit for bit (a zero's sign aside) whenever the largest high
+// word of the values named below stays under HI_INF; otherwise the caller repeats
+// the substep full width.  The Gauss-Jordan inverse of a Katz96 substep (blocks of
+// 2 and 3) then takes 12 divisions instead of the full width's 50, and its row
+// operations are those inside the blocks instead of 20 of 10 elements; the LU takes
+// one pivot comparison per column.
 constexpr int HI_INF = 0x7ff00000;
 __device__ __forceinline__ int mag_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
 
