@@ -550,11 +550,11 @@ def run_main(args, wl, desc):
     # DRAM bytes per launch from an ncu capture of the same kernel on a
     # smaller batch, scaled by systems (every system's network and state cross
     # HBM once per launch, so traffic grows in proportion to the systems):
-    # k_lu on 1,776 dense systems read 10.1 MB (5,694 B per system against
+    # k_lu on 1,776 dense systems read 9.64 MB (5,430 B per system against
     # 5,376 B of network and state; its state writes were still in L2 when the
     # capture ended), k_lane LU_F64 on 16,384 Katz96 cells 136.7 B
     traffic_per_system = args.traffic_per_system or {
-        ("dense", "lu_f64"): 5694.0, ("katz96", "lu_f64"): 136.7}.get((args.workload, main_solver), 0.0)
+        ("dense", "lu_f64"): 5430.0, ("katz96", "lu_f64"): 136.7}.get((args.workload, main_solver), 0.0)
     traffic = traffic_per_system * S / len(bounds) if traffic_per_system else None
     roof = {"bound": "fp32" if fp32_main else "fp64", "achieved": achieved, "peak": peak,
             "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
