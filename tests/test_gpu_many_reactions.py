@@ -82,3 +82,20 @@ def test_staging_does_not_outweigh_an_attempt(cuda_device):
                           device_arrays=arrays)
             best[solver] = min(best.get(solver, 1e9), time.perf_counter() - t)
     assert best["lu_f64"] <= 3.0 * best["mixed"], best
+
+
+@pytest.mark.parametrize("solver", ["auto", "gje_f64"])
+@pytest.mark.parametrize("n,react", [(16, 300), (16, 301), (32, 384), (32, 385)])
+def test_batch_staging_on_both_sides_of_the_rule(cuda_device, n, react, solver):
+    """A group's result in a batch, staged either way, is the one of the call of
+    its own: bit for bit for Gauss-Jordan, within the plain FP64 path's bound for
+    the LU."""
+    net, y0 = _net(n, 6, react, 10)
+    alone = y0.copy()
+    _, st, steps = lib.integrate(net, alone, 0.0, 1e-4, 1e-5, 1e-3, "sie", solver, "gold")
+    (y, s, c), = lib.integrate_batch([W.Workload(net, y0, 0.0, 1e-4, 1e-5, 1e-3)], "sie", solver, "gold")
+    assert np.array_equal(s, st) and np.array_equal(c, steps)
+    if solver == "gje_f64":
+        assert np.array_equal(y, alone)
+    else:
+        assert mixed_err(y, alone, 1e-5) <= 1e-10

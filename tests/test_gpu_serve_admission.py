@@ -27,12 +27,12 @@ def test_records_do_not_narrow_admission(cuda_device):
     run side by side under a budget that holds their arrays only."""
     a, b = _slow(1), _slow(2)
     with serve.Server(solver="auto", hbm_budget_bytes=_bytes(a) + _bytes(b), max_inflight=4) as srv:
+        deadline = time.time() + 60.0
         ia = srv.submit(a)
-        while srv.stats()["running"] < 1:
+        while srv.stats()["running"] < 1 and time.time() < deadline:
             time.sleep(1e-4)
         ib = srv.submit(b)
         both = False
-        deadline = time.time() + 60.0
         while not both and time.time() < deadline:
             s = srv.stats()
             both = s["running"] == 2 and s["resident_bytes"] == _bytes(a) + _bytes(b)
@@ -53,7 +53,8 @@ def test_records_are_counted_while_they_are_held(cuda_device):
     with serve.Server(solver="auto", hbm_budget_bytes=budget) as srv:
         ia = srv.submit(a)
         peak = 0
-        while srv.stats()["completed"] == 0:
+        deadline = time.time() + 60.0
+        while srv.stats()["completed"] == 0 and time.time() < deadline:
             peak = max(peak, srv.stats()["resident_bytes"])
         srv.poll(ia, 300.0)
         assert _bytes(a) < peak <= budget // 2

@@ -28,7 +28,7 @@ FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
 
 # translation units of libwind.so
 UNITS = ["api", "batch", "noalloc", "dispatch_lane", "dispatch_team", "dispatch_team8",
-         "dispatch_team16", "dispatch_team32", "dispatch_warp", "dispatch_lu", "dispatch_cta", "dispatch_mixed", "server", "global",
+         "dispatch_team16", "dispatch_team32", "dispatch_warp", "dispatch_lu", "dispatch_cta", "dispatch_mixed", "dispatch_mixed_counted", "server", "global",
          "dispatch_tile", "plugin", "dispatch_sim"]
 
 # Kernel sources the runtime plug-ins compile with NVRTC (csrc/plugin.cu),

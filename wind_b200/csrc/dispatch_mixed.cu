@@ -10,28 +10,7 @@
 
 namespace wind {
 
-using MixedFn = void (*)(const KParams*, const int*, int, double*, size_t, int);
-
-template <int METHOD, int CTRL>
-static MixedFn mixed_by_solver(int solver) {
-    if constexpr (METHOD == WIND_METHOD_RK2) return k_mixed<METHOD, CTRL, WIND_SOLVER_LU_F64>;
-    else {
-        switch (solver) {
-        case WIND_SOLVER_GJE_F64: return k_mixed<METHOD, CTRL, WIND_SOLVER_GJE_F64>;
-        case WIND_SOLVER_LU_F64: return k_mixed<METHOD, CTRL, WIND_SOLVER_LU_F64>;
-        case WIND_SOLVER_AUTO: return k_mixed<METHOD, CTRL, WIND_SOLVER_MIXED, WIND_SOLVER_LU_F64>;
-        default: return k_mixed<METHOD, CTRL, WIND_SOLVER_MIXED>;
-        }
-    }
-}
-
-static MixedFn mixed_fn(int method, int ctrl, int solver) {
-    if (method == WIND_METHOD_SIE)
-        return ctrl == WIND_CTRL_GOLD ? mixed_by_solver<WIND_METHOD_SIE, WIND_CTRL_GOLD>(solver)
-                                      : mixed_by_solver<WIND_METHOD_SIE, WIND_CTRL_DEVICE>(solver);
-    return ctrl == WIND_CTRL_GOLD ? mixed_by_solver<WIND_METHOD_RK2, WIND_CTRL_GOLD>(solver)
-                                  : mixed_by_solver<WIND_METHOD_RK2, WIND_CTRL_DEVICE>(solver);
-}
+MixedFn mixed_fn_counted(int method, int ctrl, int solver);  // dispatch_mixed_counted.cu
 
 static int nmax_of(int n) { return n <= 8 ? 8 : (n <= 16 ? 16 : 32); }
 bool team_admitted(int n, int R, bool lin, bool lists, int teams, size_t budget);
@@ -48,9 +27,11 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
     cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cap -= 1024;
     size_t smem = 0, gslot = 0, gneed = 0;
+    bool counted = false;
     for (const KParams& p : ps) {
         // the solver each group runs (AUTO: MIXED above 32 species, LU_F64 below)
         const int gs = resolve_solver(solver, p.kind, p.n_eq);
+        counted = counted || mixed_counted(p.n_eq, p.n_react);
         if (p.n_eq > 32) {
             const CtaLayout lay(p.n_eq, p.n_react, p.linear != nullptr, gs, cap, false,
                                 o.method == WIND_METHOD_SIE);
@@ -80,7 +61,10 @@ wind_status launch_mixed(const wind_options& o, const std::vector<KParams>& ps, 
         }
     }
     if (smem > (size_t)cap) return WIND_ERR_UNSUPPORTED;
-    MixedFn fn = mixed_fn(o.method, o.controller, o.solver);
+    // (the MIXED team kernel has lists of its own)
+    counted = counted && !(o.method == WIND_METHOD_SIE && o.solver == WIND_SOLVER_MIXED);
+    const MixedFn fn = counted ? mixed_fn_counted(o.method, o.controller, o.solver)
+                               : mixed_fn<false>(o.method, o.controller, o.solver);
     if (allow_block_smem((const void*)fn) != cudaSuccess)
         return launch_status("k_mixed shared-memory attribute");
     int nb = 0;

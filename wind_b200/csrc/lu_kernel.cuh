@@ -498,6 +498,88 @@ __device__ __noinline__ bool lu_stage_apart(unsigned mask, int l, int N, int R, 
     return lu_stage<L, COLS, 4>(mask, l, N, R, k_in, sp, Lg, base, sorted);
 }
 
+// The same with every lane looking through all reactions and walking its list once
+// per column, for k_mixed on networks of few reactions (mixed_counted): system s's
+// rates, the dense term transposed, the incidence lists and the Jacobian terms.  A species index >= N marks the system BAD_INPUT
+// (returned) and nothing of it is read again.
+template <int L, int COLS>
+__device__ __forceinline__ bool lu_stage_scan(const LuCtx<L, COLS>& c, const KParams& p, int64_t s, double* rates,
+                                              int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, double* LT) {
+    const int N = c.N, R = p.n_react, l = c.l;
+    const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * R;
+    bool bad = false;
+    for (int r = l; r < R; r += L) {
+        const double k = p.rates[s * R + r];
+        const uint2 q = __ldg(sp + r);
+        // the reactants' s is -2 where they are one species that is not made
+        // again, the products' +2 where they are one that is not consumed
+        const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+        rates[2 * r] = (double)min(-1, stoich(a, a, b, cc, d)) * k;
+        rates[2 * r + 1] = (double)max(1, stoich(cc, a, b, cc, d)) * k;
+        const unsigned nn = (unsigned)N;
+        bad = bad || (q.x & 0xffffu) >= nn || (q.x >> 16) >= nn || (q.y & 0xffffu) >= nn || (q.y >> 16) >= nn;
+    }
+    if (__any_sync(c.mask, bad)) return true;
+    for (int j = l; j < N; j += L) {
+        int cnt = 0, terms = 0;
+        for (int r = 0; r < R; r++) {
+            const uint2 q = __ldg(sp + r);
+            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+            cnt += (a == j) | (b == j) | (cc == j) | (d == j);
+            terms += stoich(j, a, b, cc, d) ? 2 : 0;
+        }
+        inc_off[j + 1] = (cnt + 3) & ~3;
+        term_off[j + 1] = (terms + 3) & ~3;
+    }
+    __syncwarp(c.mask);
+    if (l == 0) {
+        inc_off[0] = term_off[0] = 0;
+        for (int j = 0; j < N; j++) {
+            inc_off[j + 1] += inc_off[j];
+            term_off[j + 1] += term_off[j];
+        }
+        rates[2 * R] = 0.0;
+        rates[2 * R + 1] = __longlong_as_double(0x7ff8000000000000ll);
+        c.vb[COLS] = 0.0;
+    }
+    __syncwarp(c.mask);
+    for (int j = l; j < N; j += L) {
+        int o = inc_off[j];
+        for (int r = 0; r < R; r++) {
+            const uint2 q = __ldg(sp + r);
+            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+            if (a != j && b != j && cc != j && d != j) continue;
+            const int st = stoich(j, a, b, cc, d);
+            int slot = st < 0 ? 2 * r : 2 * r + 1;
+            if (st == 0) slot = finite64(rates[2 * r]) || finite64(rates[2 * r + 1]) ? 2 * R : 2 * R + 1;  // 0 * k
+            inc[o++] = rx_pack(slot, a, b);
+        }
+        // d w / d y_a = k y_b, then d w / d y_b = k y_a, per column in list order
+        const int e0 = inc_off[j];
+        int t = term_off[j];
+        for (int col = 0; col < N; col++) {
+            const int t0 = t;
+            for (int e = e0; e < o; e++) {
+                const uint32_t q = inc[e];
+                const int slot = (int)(q & 0x7ffffu) >> 3, a = (int)(rx_first(q) >> 3), b = (int)(rx_second(q) >> 3);
+                if (slot >= 2 * R) continue;
+                if (a == col) term[t++] = rx_pack(slot, b, col);
+                if (b == col) term[t++] = rx_pack(slot, a, col);
+            }
+            if (t > t0) term[t - 1] |= RX_MARK;
+        }
+        // padding: rate zero, the zero beside the state, the column beside the row
+        while (o < inc_off[j + 1]) inc[o++] = rx_pack(2 * R, COLS, COLS);
+        while (t < term_off[j + 1]) term[t++] = rx_pack(2 * R, COLS, COLS);
+        if (LT) {
+            const float* Lg = p.linear + s * (int64_t)N * N;
+            for (int k = 0; k < N; k++) LT[k * N + j] = Lg[j * N + k];
+        }
+    }
+    __syncwarp(c.mask);
+    return false;
+}
+
 // Warps per SM the registers are planned for.  8 (250 registers at 32 columns)
 // and 10 or 12 (200, 168) measured alike on 3,000 dense systems of 32 species
 // (696, 682, 701 ms); alone on an SM a substep takes 6.0 us with 8, 7.1 us with
@@ -508,7 +590,7 @@ constexpr int LU_BLOCKS = 8;
 // every warp (of the block's first `teams` teams) take tickets from the group's
 // queue until it is empty.  `smem_raw` holds `teams` team slices, laid out with or
 // without the sorted Jacobian terms (GUARD: with).
-template <int L, int COLS, bool GUARD, int CTRL>
+template <int L, int COLS, bool GUARD, int CTRL, bool COUNTED>
 __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw, int teams, int tpw, bool sorted) {
     using Ctx = LuCtx<L, COLS>;
     constexpr int CAP = Cap<WIND_METHOD_SIE, CTRL>::value;
@@ -531,12 +613,18 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
     c.live = false;
     c.N = p.n_eq;
     unsigned char* base = smem_raw + team * lay.bytes;
-    c.rates = reinterpret_cast<double*>(base + lay.rates);
-    c.inc_off = reinterpret_cast<int*>(base + lay.inc_off);
-    c.inc = reinterpret_cast<uint32_t*>(base + lay.inc);
-    c.term_off = reinterpret_cast<int*>(base + lay.term_off);
-    c.term = sorted ? reinterpret_cast<uint32_t*>(base + lay.term) : nullptr;
-    c.LT = lin ? reinterpret_cast<double*>(base + lay.lt) : nullptr;
+    double* rates = reinterpret_cast<double*>(base + lay.rates);
+    int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
+    uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
+    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
+    uint32_t* term = sorted ? reinterpret_cast<uint32_t*>(base + lay.term) : nullptr;
+    double* LT = lin ? reinterpret_cast<double*>(base + lay.lt) : nullptr;
+    c.rates = rates;
+    c.inc_off = inc_off;
+    c.inc = inc;
+    c.term_off = term_off;
+    c.term = term;
+    c.LT = LT;
     c.vb = reinterpret_cast<double*>(base + lay.vb);
     double* rows = reinterpret_cast<double*>(base + lay.rows);
     double* rows2 = reinterpret_cast<double*>(base + lay.rows2);
@@ -568,11 +656,15 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
                     phase = FULL;  // no system left: idle turns from here on
                     break;
                 }
-                const double* k = p.rates + s * p.n_react;
-                const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * p.n_react;
-                const float* Lg = lin ? p.linear + s * (int64_t)N * N : nullptr;
-                stop = GUARD ? lu_stage<L, COLS, 1>(c.mask, l, N, p.n_react, k, sp, Lg, base, true)
-                             : lu_stage_apart<L, COLS>(c.mask, l, N, p.n_react, k, sp, Lg, base, sorted);
+                if constexpr (COUNTED) {
+                    const double* k = p.rates + s * p.n_react;
+                    const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * p.n_react;
+                    const float* Lg = lin ? p.linear + s * (int64_t)N * N : nullptr;
+                    stop = GUARD ? lu_stage<L, COLS, 1>(c.mask, l, N, p.n_react, k, sp, Lg, base, true)
+                                 : lu_stage_apart<L, COLS>(c.mask, l, N, p.n_react, k, sp, Lg, base, sorted);
+                } else {
+                    stop = lu_stage_scan(c, p, s, rates, inc_off, inc, term_off, term, LT);
+                }
                 st = stop ? WIND_SYS_BAD_INPUT : WIND_SYS_OK;
                 y = (l < N) ? p.y[s * N + l] : 0.0;
                 tnow = p.tnow;
@@ -687,7 +779,7 @@ __device__ __forceinline__ void lu_run(const KParams& p, unsigned char* smem_raw
 template <int L, int COLS, int CTRL>
 __global__ void __launch_bounds__(32, LU_BLOCKS) k_lu(const KParams p, int tpw, int sorted) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    lu_run<L, COLS, false, CTRL>(p, smem_raw, tpw, tpw, sorted != 0);
+    lu_run<L, COLS, false, CTRL, true>(p, smem_raw, tpw, tpw, sorted != 0);
 }
 
 }  // namespace wind

@@ -39,8 +39,8 @@ __device__ __forceinline__ int rx_scan(unsigned mask, int l, int v) {
 // every lane then lists its own marks.  (With every lane looking through all the
 // reactions, a reaction cost some 200 cycles and pass.)
 template <int L>
-__device__ __noinline__ int rx_list(unsigned mask, int l, int N, int R, const uint2* sp, uint32_t* touched,
-                                    uint32_t* out) {
+__device__ __forceinline__ int rx_list(unsigned mask, int l, int N, int R, const uint2* sp, uint32_t* touched,
+                                       uint32_t* out) {
     int cnt = 0;
     constexpr int PER = 32 / L;
     uint2 next[PER];

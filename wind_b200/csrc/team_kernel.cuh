@@ -493,10 +493,92 @@ __device__ __forceinline__ bool team_stage(unsigned mask, int l, int N, int R, c
     return false;
 }
 
+// The same with every lane looking through all reactions and walking its list once
+// per column, for k_mixed on networks of few reactions (mixed_counted): system s's
+// signed rates, the dense term transposed, the unit lists and, with JAC, the
+// Jacobian terms.  A species index >= N marks the system BAD_INPUT
+// (returned) and nothing of it is read again.
+template <int NMAX, bool JAC>
+__device__ __forceinline__ bool team_stage_scan(const TeamCtx<NMAX>& c, const KParams& p, int64_t s, double* rates,
+                                                int* inc_off, uint32_t* inc, int* term_off, uint32_t* term, float* LT) {
+    const int N = c.N, R = p.n_react, l = c.l;
+    const uint2* sp = reinterpret_cast<const uint2*>(p.species) + s * R;
+    bool bad = false;
+    for (int r = l; r < R; r += NMAX) {
+        const double k = p.rates[s * R + r];
+        rates[2 * r] = -k;
+        rates[2 * r + 1] = k;
+        const uint2 q = __ldg(sp + r);
+        const unsigned nn = (unsigned)N;
+        bad = bad || (q.x & 0xffffu) >= nn || (q.x >> 16) >= nn || (q.y & 0xffffu) >= nn || (q.y >> 16) >= nn;
+    }
+    if (__any_sync(c.mask, bad)) return true;
+    // units of species l in reaction (a, b -> cc, d): nn times -, then np times +
+    if (l < N) {
+        int cnt = 0;
+        for (int r = 0; r < R; r++) {
+            const uint2 q = __ldg(sp + r);
+            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+            cnt += (a == l) + (b == l) + (cc == l) + (d == l);
+        }
+        inc_off[l + 1] = (cnt + 3) & ~3;
+        if (JAC) term_off[l + 1] = (2 * cnt + 3) & ~3;
+    }
+    team_sync(c.mask);
+    if (l == 0) {
+        inc_off[0] = 0;
+        for (int j = 0; j < N; j++) inc_off[j + 1] += inc_off[j];
+        if (JAC) {
+            term_off[0] = 0;
+            for (int j = 0; j < N; j++) term_off[j + 1] += term_off[j];
+        }
+        rates[2 * R] = 0.0;
+        c.v[NMAX] = 0.0;
+    }
+    team_sync(c.mask);
+    if (l < N) {
+        int o = inc_off[l];
+        for (int r = 0; r < R; r++) {
+            const uint2 q = __ldg(sp + r);
+            const int a = q.x & 0xffff, b = q.x >> 16, cc = q.y & 0xffff, d = q.y >> 16;
+            const int nn = (a == l) + (b == l), np = (cc == l) + (d == l);
+            for (int u = 0; u < nn + np; u++) inc[o++] = rx_pack(2 * r + (u >= nn), a, b);
+        }
+        if (JAC) {
+            // d w / d y_a = k y_b, then d w / d y_b = k y_a: per reaction all
+            // units of the first before the second
+            int t = term_off[l];
+            for (int col = 0; col < N; col++) {
+                const int t0 = t;
+                for (int e = inc_off[l]; e < o;) {
+                    const uint32_t q = inc[e];
+                    const int r = (int)(q & 0x7ffffu) >> 4, a = (int)(rx_first(q) >> 3), b = (int)(rx_second(q) >> 3);
+                    int n = e + 1;  // the reaction's units are neighbours
+                    while (n < o && ((int)(inc[n] & 0x7ffffu) >> 4) == r) n++;
+                    if (a == col)
+                        for (int u = e; u < n; u++) term[t++] = rx_pack((int)(inc[u] & 0x7ffffu) >> 3, b, col);
+                    if (b == col)
+                        for (int u = e; u < n; u++) term[t++] = rx_pack((int)(inc[u] & 0x7ffffu) >> 3, a, col);
+                    e = n;
+                }
+                if (t > t0) term[t0] |= RX_MARK;
+            }
+            while (t < term_off[l + 1]) term[t++] = rx_pack(2 * R, NMAX, NMAX) | RX_MARK;
+        }
+        while (o < inc_off[l + 1]) inc[o++] = rx_pack(2 * R, NMAX, NMAX);
+        if (LT) {
+            const float* Lg = p.linear + s * (int64_t)N * N;
+            for (int k = 0; k < N; k++) LT[k * NMAX + l] = Lg[l * N + k];
+        }
+    }
+    team_sync(c.mask);
+    return false;
+}
+
 // The persistent team loop over one group's systems: the first `tpw` teams of
 // every warp (of the block's first `teams` teams) take tickets from the group's
 // queue until it is empty.  `smem_raw` holds `teams` team slices.
-template <int NMAX, int METHOD, int CTRL>
+template <int NMAX, int METHOD, int CTRL, bool COUNTED>
 __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_raw, int teams, int tpw) {
     constexpr int CAP = Cap<METHOD, CTRL>::value;
     constexpr bool SIE = METHOD == WIND_METHOD_SIE;
@@ -515,12 +597,18 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
     c.w = reinterpret_cast<double*>(base + lay.w);
     c.v = reinterpret_cast<double*>(base + lay.vec);
     c.f = c.v + NMAX + 2;
-    c.LT = lin ? reinterpret_cast<float*>(base + lay.lt) : nullptr;
-    c.rates = reinterpret_cast<double*>(base + lay.rates);
-    c.inc_off = reinterpret_cast<int*>(base + lay.inc_off);
-    c.inc = reinterpret_cast<uint32_t*>(base + lay.inc);
-    c.term_off = reinterpret_cast<int*>(base + lay.term_off);
-    c.term = reinterpret_cast<uint32_t*>(base + lay.term);
+    float* LT = lin ? reinterpret_cast<float*>(base + lay.lt) : nullptr;
+    double* rates = reinterpret_cast<double*>(base + lay.rates);
+    int* inc_off = reinterpret_cast<int*>(base + lay.inc_off);
+    uint32_t* inc = reinterpret_cast<uint32_t*>(base + lay.inc);
+    c.LT = LT;
+    c.rates = rates;
+    c.inc_off = inc_off;
+    c.inc = inc;
+    int* term_off = reinterpret_cast<int*>(base + lay.term_off);
+    uint32_t* term = reinterpret_cast<uint32_t*>(base + lay.term);
+    c.term_off = term_off;
+    c.term = term;
     const int N = c.N, l = c.l;
     const uint64_t t_start = p.timeout_ns ? global_ns() : 0;
     const double tend = p.tend;
@@ -543,9 +631,12 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
                 if (l == 0) ticket = atomicAdd(&p.counters[CNT_QUEUE], 1ull);
                 s = (int64_t)__shfl_sync(c.mask, ticket, c.leader);
                 if (s >= p.nsys) return;
-                stop = team_stage<NMAX, SIE>(c.mask, l, N, p.n_react, p.rates + s * p.n_react,
-                                             reinterpret_cast<const uint2*>(p.species) + s * p.n_react,
-                                             lin ? p.linear + s * (int64_t)N * N : nullptr, base);
+                if constexpr (COUNTED)
+                    stop = team_stage<NMAX, SIE>(c.mask, l, N, p.n_react, p.rates + s * p.n_react,
+                                                 reinterpret_cast<const uint2*>(p.species) + s * p.n_react,
+                                                 lin ? p.linear + s * (int64_t)N * N : nullptr, base);
+                else
+                    stop = team_stage_scan<NMAX, SIE>(c, p, s, rates, inc_off, inc, term_off, term, LT);
                 st = stop ? WIND_SYS_BAD_INPUT : WIND_SYS_OK;
                 y = (l < N) ? p.y[s * N + l] : 0.0;
                 tnow = p.tnow;
@@ -659,7 +750,7 @@ __device__ __forceinline__ void team_run(const KParams& p, unsigned char* smem_r
 template <int NMAX, int METHOD, int CTRL>
 __global__ void __launch_bounds__(32) k_team(const KParams p, int tpw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    team_run<NMAX, METHOD, CTRL>(p, smem_raw, tpw, tpw);
+    team_run<NMAX, METHOD, CTRL, true>(p, smem_raw, tpw, tpw);
 }
 
 }  // namespace wind
