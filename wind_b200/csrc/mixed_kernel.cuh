@@ -29,8 +29,8 @@ __host__ __device__ inline int mixed_teams(int nmax, int team_bytes, int smem_ca
 
 // Whether a group's systems are staged by counting, a reaction per lane, or with
 // every lane looking through all reactions.  Counting wins by the reaction: one
-// attempt of 4,000 systems takes 2.75 ms by looking and 1.0 by counting with 32
-// species and 640 reactions, 0.83 and 0.68 with 16 and 320.  But the LU of up to 16
+// attempt of 4,000 systems takes 2.75 ms by looking and 0.68 by counting with 32
+// species and 640 reactions, 0.83 and 0.28 with 16 and 320.  But the LU of up to 16
 // species and RK2 run slower in the kernel that has the counting beside them (40
 // attempts of 8 species and 200 reactions: 1.71 and 2.68 ms, of 16 and 160: 1.81 and
 // 2.88; the RK2 batch of 1,000 mixed sizes 1.79 and 2.46), so where looking costs
